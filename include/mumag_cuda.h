@@ -282,9 +282,11 @@ int mm_minimize_dev(mm_problem* h, const double* B_ext, double* d_m_inout, doubl
 #define MM_KERNEL_HESSIAN 3  /* local Hessian action over the magnetic rows               */
 int mm_time_kernel(mm_problem* h, int kernel, int reps, double* ms_per_launch, double* bytes_per_launch);
 
-/* Solver options.  MM_OPT_GRAPH (default 1): run the PCG iterations inside a CUDA graph whose
- * conditional WHILE node loops on the device until convergence; 0 polls the device flag from the
- * host every four iterations (same kernels, same results). */
+/* Solver options.  MM_OPT_GRAPH (default 1): run a demag solve on the device until convergence: as one
+ * persistent launch (multilevel preconditioners; FP32 V-cycles up to 786,432 nodes; fewer than four solves or
+ * minimizations in flight on the device), else as separate kernels inside a CUDA graph whose conditional WHILE
+ * node loops; 0 polls the device flag from the host every four iterations (separate kernels).  The same
+ * results either way, bit for bit. */
 #define MM_OPT_GRAPH 1
 /* MM_OPT_PRECISION (before mm_build_poisson): MM_PRECISION_FP64 (default) is the reference's plain
  * FP64 PCG; MM_PRECISION_MIXED keeps U, the right-hand side and the true residual in FP64 and solves
@@ -313,15 +315,16 @@ int mm_time_kernel(mm_problem* h, int kernel, int reps, double* ms_per_launch, d
  * kernel is scheduled while its predecessor drains (every solver kernel waits for its predecessor's
  * results at entry); 0 launches them normally.  Same results either way. */
 #define MM_OPT_PDL 8
-/* MM_OPT_COARSE_FUSE (bit mask, default 1): with 3 or more levels, at most 256 rows on the coarsest
+/* MM_OPT_COARSE_FUSE (bit mask, default 3): with 3 or more levels, at most 256 rows on the coarsest
  * level and at most 4Mi entries in the n(L-2) x n(L-1) dense factors (so that they cost little memory
  * and host setup time), the two coarsest levels of the V-cycle (level L-2's residual, restriction,
  * the dense coarsest solve, prolongation and post-smoothing: five dependent kernels) run as two
  * kernels applying the same linear map in factored form, x2 = T b + W (Z b) with T = 2S - S A S,
  * W = (I - S A) P and Z = Ainv R (I - A S) (S the smoother diagonal; T sparse with A's pattern, W and Z
  * dense, formed at mm_build_poisson).  Bit 0: in the FP64 solver, bit 1: in the FP32 solver of the
- * mixed method.  Same V-cycle up to summation order.  (80 nm cube on GB300: the FP64 solve 7 % faster,
- * the FP32 iteration unchanged; mm_autotune measures it per problem.) */
+ * mixed and FP32-preconditioned methods.  Same V-cycle up to summation order.  (80 nm cube on GB300: the FP64
+ * solve 7 % faster as separate kernels; the FP32 V-cycle of the one-launch PCG takes 31k clocks on these levels
+ * against 55k; mm_autotune measures it per problem.) */
 #define MM_OPT_COARSE_FUSE 9
 /* MM_OPT_MIN_FP32: precision of the minimizer's inner preconditioner solve (the Steihaug PCG on the
  * local Hessian P y = g of mm_minimize).  -1 (default) follows MM_OPT_PRECISION: FP32 entries, vectors
@@ -360,7 +363,8 @@ int mm_time_kernel(mm_problem* h, int kernel, int reps, double* ms_per_launch, d
 /* MM_OPT_COARSE_CYCLE (bit mask, default 0; mm_autotune keeps what is faster): with four levels, the
  * fused restriction at level 1 and the fused coarse correction, the V-cycle runs levels 1 .. 3 (the
  * level-1 restriction, both coarse-correction phases, the level-1 prolongation and post-smoothing)
- * in one cooperative launch with grid barriers instead of five launches; bit-identical results.
+ * in one cooperative launch with grid barriers instead of five launches; bit-identical results.  Concerns
+ * the separate kernels only.
  * Bit 0 the FP64 solver, bit 1 the FP32 solver. */
 #define MM_OPT_COARSE_CYCLE 16
 /* MM_OPT_CSR_LANES (after mm_build_poisson): every compressed-row operator of the hierarchy (coarse
@@ -385,7 +389,7 @@ int mm_get_option(mm_problem* h, int option, int* value);
 
 /* Autotuner (after mm_build_poisson): for every compressed-row operator of the hierarchy (coarse levels,
  * restrictions, prolongations; both precisions) tries 2, 4, 8, 16 and 32 lanes per row, each timed as
- * whole V-cycles so that cache state and neighbouring kernels are those of a solve, and keeps the
+ * PCG iterations or whole V-cycles so that cache state and neighbours are those of a solve, and keeps the
  * fastest when it beats the heuristic's shape by more than 3 %; then times the V-cycle with and without the fused coarse correction in each solver and
  * sets MM_OPT_COARSE_FUSE accordingly.  CUDA events on the problem's stream, `reps`
  * launches per candidate.  A JSON report (candidates, times in microseconds, choices) is written to

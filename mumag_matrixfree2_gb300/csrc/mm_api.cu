@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -16,6 +17,7 @@
 
 #include "../../include/mumag_cuda.h"
 #include "mm_kernels.cuh"
+#include "mm_pcg.cuh"
 #include "mm_setup.h"
 
 using mmk::BS;
@@ -59,6 +61,9 @@ inline int grid_ilp(int64_t n) {
   const int64_t per = (int64_t)BS * mmk::ILP;
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + per - 1) / per, g_elem_cap));
 }
+// warps (log2) of one chunk of the PCG's reductions over n rows (chunk_finish): one warp while the rows
+// give every SM fewer than 16 of them, else the block's eight
+inline int red_kshift(int64_t n) { return grid_ilp(n) * (BS / 32) < 2432 ? 0 : 3; }
 inline int grid_rows(int64_t n, int tpr) {
   const int rpb = BS / tpr;
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + rpb - 1) / rpb, MAXG));
@@ -127,14 +132,45 @@ struct SolverT {
   int sms = 0;
 };
 
-// Layout choice: one thread per row when the rows alone fill the GPU (>= 64Ki rows), else enough
-// lanes per row to reach ~256Ki threads, capped by the average row length.
-int choose_tpr(int64_t rows, int64_t nnz) {
+// Sizes whose PCG runs as one launch (V-cycle in T).  FP64: all measured (1,331 to 1,601,613 rows: 316 against
+// 469 us, 6.24 against 6.69 ms a solve).  FP32: up to 3/4 Mi rows (357,911 rows 1.68 against 1.78 ms; 1,601,613
+// rows 5.17 against 4.96 ms: streaming FP32 operators wants the 2048 threads an SM of the separate kernels).
+template <class T>
+bool one_launch_rows(int64_t n) {
+  return sizeof(T) == 8 || n <= 786432;
+}
+
+// Layout choice for an operator of an n-row problem: one thread per row from 64Ki rows on, else t lanes per row
+// (2..32) by the cost of a phase of the one-launch PCG on an SM in clocks: its warp instructions (an FP64 one
+// holds the SM's FP64 pipe for 16 clocks, so a row's log2 t reduction steps cost as much as its entries: 32
+// lanes on the 62-entry rows of the 40 nm cube's level-0 fused restriction spend 7 a row, 4 lanes 2.25) against
+// the latency of its dependent loads (~1400 clocks for each eight entries of a lane), which overlap in part.
+// FP32 V-cycle, a solve with it and with lanes for ~256Ki threads: 40 nm cube 700 and 799 us, 80 nm cube 1.68 and
+// 1.79 ms.  The separate kernels of larger FP32 problems want the latter.
+template <class T>
+int choose_tpr(int64_t rows, int64_t nnz, int64_t n) {
   if (rows >= 65536) return 1;
   const double avg = rows > 0 ? (double)nnz / (double)rows : 1.0;
-  int t = 2;
-  while (t < 32 && (rows * t < 262144) && t < avg) t *= 2;
-  return t;
+  if (!one_launch_rows<T>(n)) {
+    int t = 2;
+    while (t < 32 && (rows * t < 262144) && t < avg) t *= 2;
+    return t;
+  }
+  const double per_sm = (double)rows / 152.0;
+  const double clocks = sizeof(T) == 8 ? 16.0 : 3.0;  // a warp's multiply-add or reduction step
+  int best = 2;
+  double best_cost = 1e300;
+  for (int t = 2, lg = 1; t <= 32; t *= 2, ++lg) {
+    const double warps = std::ceil(per_sm * t / 32.0), each = std::ceil(avg / t);
+    const double pipe = warps * (each + lg) * clocks;
+    const double wait = std::ceil(warps / 24.0) * std::ceil(each / 8.0) * 1400.0;
+    const double cost = std::max(pipe, wait) + 0.3 * std::min(pipe, wait);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = t;
+    }
+  }
+  return best;
 }
 
 thread_local std::string g_create_error;
@@ -238,12 +274,15 @@ struct mm_problem {
   double *d_b = nullptr, *d_x = nullptr, *d_r64 = nullptr;
   float *d_r32 = nullptr, *d_d32 = nullptr;
   double* d_part = nullptr;      // NRED x MAXG block partials (shared by every reduction)
+  mmk::PBar* d_pbar = nullptr;   // the one-launch PCG's grid barrier
+  int coop_sms = 0;              // SMs a cooperative launch can fill (0: not supported)
+  int pcg_cap = 0;               // blocks of the one-launch PCG at most in this call (SolveScope)
   mmk::Scalars* d_sc = nullptr;  // scalars of the FP64 solver, the energy and the minimizer
   mmk::Scalars* d_sc32 = nullptr;
   mmk::Scalars* h_sc = nullptr;  // pinned
   bool use_graph = true;
   bool pdl = true;               // MM_OPT_PDL
-  int coarse_fuse = 1;           // MM_OPT_COARSE_FUSE: bit 0 the FP64 solver, bit 1 the FP32 solver
+  int coarse_fuse = 3;           // MM_OPT_COARSE_FUSE: bit 0 the FP64 solver, bit 1 the FP32 solver
   int fuse_restrict = 3;         // MM_OPT_FUSE_RESTRICT: bit 0 the FP64 solver, bit 1 the FP32 solver
   int coarse_cycle = 0;          // MM_OPT_COARSE_CYCLE: bit 0 the FP64 solver, bit 1 the FP32 solver
   int sa_theta_e3 = 0;           // MM_OPT_SA_THETA_E3 (0: the setup's default)
@@ -518,7 +557,7 @@ struct mm_problem {
   // lanes-per-row kernels.
   template <class T>
   DevMatT<T> upload_mat(const mm::HostCSR& A, bool force_sell = false) {
-    const int tpr = force_sell ? 1 : choose_tpr(A.n_rows, A.nnz());
+    const int tpr = force_sell ? 1 : choose_tpr<T>(A.n_rows, A.nnz(), N);
     DevMatT<T> d;
     d.tpr = tpr;
     d.nnz = A.nnz();
@@ -836,7 +875,8 @@ void enqueue_vcycle(mm_problem* h, SolverT<T>& S, const T* r, T* z, bool in_loop
               [&] { spmv<3, T>(h, c.P, lv[l + 1].x2, c.x, nullptr, c.x, done); });  // x += P e
     if (l == 0) {
       tagged<T>(h, MM_PROF_SMOOTH0, 0, mat_bytes(c.A) + 4.0 * w * c.n, [&] {
-        launch(h, mmk::k_smooth_dot<T>, grid_ilp(c.n), BS, c.A.s, c.x, r, c.s, z, sc, h->d_part, done, z64);
+        launch(h, mmk::k_smooth_dot<T>, grid_ilp(c.n), BS, c.A.s, c.x, r, c.s, z, sc, h->d_part, done, z64,
+               red_kshift(c.n));
         LAUNCH_CHECK();
       });
     } else {
@@ -882,13 +922,14 @@ void enqueue_dir_step(mm_problem* h, SolverT<T>& S) {
   const double w = sizeof(T);
   auto& l0 = S.lv[0];
   tagged<T>(h, MM_PROF_PCG_DIR, 0, mat_bytes(l0.A) + 5.0 * w * N, [&] {
-    launch(h, mmk::k_pcg_dir<T>, grid_ilp(N), BS, l0.A.s, S.z, S.p, S.Ap, S.sc, h->d_part);
+    launch(h, mmk::k_pcg_dir<T>, grid_ilp(N), BS, l0.A.s, S.z, S.p, S.Ap, S.sc, h->d_part,
+           red_kshift(N));
     LAUNCH_CHECK();
   });
   const bool ml = multilevel(h, S);
   tagged<T>(h, MM_PROF_PCG_STEP, 0, (ml ? 8.0 : 6.0) * w * N, [&] {
     launch(h, mmk::k_pcg_step<T>, grid_ilp(N), BS, N, S.x, S.r, S.p, S.Ap, ml ? l0.s : nullptr, l0.x, S.sc,
-                                                        h->d_part);
+           h->d_part, red_kshift(N));
     LAUNCH_CHECK();
   });
 }
@@ -1014,6 +1055,178 @@ void finish_pcg(mm_problem* h, const PcgPending& pend, int* iters, double* r2_ou
   if (r2_out) *r2_out = h->h_sc->red[R_R2];
 }
 
+
+// ---------------------------------------------------------------------------------------------
+// The PCG as one launch (mm_pcg.cuh): S's vectors and finest operator, F's hierarchy.
+// ---------------------------------------------------------------------------------------------
+template <class T>
+mmk::POp<T> persistent_op(const DevMatT<T>& M) {
+  mmk::POp<T> o{};
+  while ((1 << o.lg) < M.tpr) ++o.lg;
+  o.n = M.tpr == 1 ? M.s.n : M.c.n;
+  o.ptr = M.tpr == 1 ? M.s.sptr : M.c.ptr;
+  o.col = M.tpr == 1 ? M.s.col : M.c.col;
+  o.val = M.tpr == 1 ? M.s.val : M.c.val;
+  return o;
+}
+
+template <class T>
+bool persistent_ok(mm_problem* h, const SolverT<T>& F) {
+  return h->use_graph && !h->prof && h->pcg_cap > 0 && multilevel(h, F) && (int)F.lv.size() <= mmk::PLEV &&
+         one_launch_rows<T>(h->N);
+}
+
+// Blocks: one per 256 rows (FP64 V-cycle: two FP64 operations a clock an SM) or 512 (FP32: the 45,570-node
+// particle takes 628 us with one per 512, 713 with one per 1024, and leaves SMs to other streams' problems),
+// at most one per SM.  Up to 16 as one cluster of 16, whose hardware barrier costs a quarter of the grid's.
+constexpr int PCG_CLUSTER = 16;
+
+template <class TV>
+int persistent_blocks(mm_problem* h) {
+  const int rows = sizeof(TV) == 8 ? 256 : 512;
+  const int want = std::min((h->N + rows - 1) / rows, h->pcg_cap);
+  return std::max(want, PCG_CLUSTER);
+}
+
+// One solve or minimization in flight.  Their number on the device decides how each runs its PCG, so that
+// several threads' problems share the GPU: alone on every SM, with one or two others on a third of them each,
+// and with more as separate kernels, whose many small launches overlap (48 particles on 16 threads, FP32
+// V-cycle: 16.3 s with every SM for each, 13.2 s with a cluster of 16 blocks each, 11.1 s as separate kernels).
+// The results are the same bits.
+std::atomic<int> g_solving[64];
+
+struct SolveScope {
+  std::atomic<int>& n;
+  explicit SolveScope(mm_problem* h) : n(g_solving[std::min(std::max(h->device, 0), 63)]) {
+    const int k = ++n;
+    h->pcg_cap = k == 1 ? h->coop_sms : k <= 3 ? h->coop_sms / 3 : 0;
+  }
+  ~SolveScope() { --n; }
+};
+
+// The arguments of the one-launch PCG; returns its blocks.
+template <class TP, class TV>
+int persistent_args(mm_problem* h, SolverT<TP>& S, SolverT<TV>& F, mmk::PcgArgs<TP, TV>& a) {
+  const int L = (int)F.lv.size();
+  const int bit = sizeof(TV) == 8 ? 0 : 1;
+  const bool use_rf = (h->fuse_restrict >> bit) & 1;
+  const bool fused = F.fused && ((h->coarse_fuse >> bit) & 1);
+  const int blocks = persistent_blocks<TV>(h);
+  a.cluster = blocks <= PCG_CLUSTER;
+  a.n = h->N;
+  a.G = grid_ilp(h->N);
+  a.Gdot = std::min(a.G, g_vec_cap);
+  a.kshift = red_kshift(h->N);
+  a.A0 = persistent_op(S.lv[0].A);
+  if constexpr (!std::is_same<TP, TV>::value) a.A0s = h->a0df;
+  a.b = S.b;
+  a.x = S.x;
+  a.r = S.r;
+  a.p = S.p;
+  a.Ap = S.Ap;
+  a.s0 = F.lv[0].s;
+  a.xv = F.lv[0].x;
+  a.rv = F.r;
+  a.z = F.z;
+  a.Z = F.Z;
+  a.zvec = F.zvec;
+  a.sc = S.sc;
+  a.part = h->d_part;
+  a.bar = h->d_pbar;
+  // the V-cycle's steps, as enqueue_vcycle launches them
+  auto add = [&](int kind, int units) -> mmk::PStep<TV>& {
+    mmk::PStep<TV>& st = a.steps[a.n_steps++];
+    st.kind = kind;
+    st.units = units;
+    return st;
+  };
+  auto rows = [&](int kind, const DevMatT<TV>& M, const TV* x, const TV* b, const TV* s, TV* y, TV* y2) {
+    const mmk::POp<TV> A = persistent_op(M);
+    const int per = A.lg == 0 ? 64 : 32 >> A.lg;
+    mmk::PStep<TV>& st = add(kind, (A.n + per - 1) / per);
+    st.A = A;
+    st.x = x;
+    st.b = b;
+    st.s = s;
+    st.y = y;
+    st.y2 = y2;
+  };
+  const int parts = (a.G * mmk::WPB) >> a.kshift;
+  add(mmk::PS_START, parts);
+  for (int l = 0; l < (fused ? L - 2 : L - 1); ++l) {
+    auto& c = F.lv[l];
+    auto& nx = F.lv[l + 1];
+    const TV* bl = l == 0 ? F.r : c.b;
+    const bool rf = use_rf && c.Rf.nnz > 0;
+    if (!rf) rows(mmk::PS_RESID, c.A, c.x, bl, nullptr, c.res, nullptr);
+    const bool no_pre = (l + 1 == L - 1) || (fused && l + 1 == L - 2);
+    rows(mmk::PS_RESTRICT, rf ? c.Rf : c.R, rf ? bl : c.res, nullptr, nx.s, nx.b, no_pre ? nullptr : nx.x);
+  }
+  if (fused) {
+    auto& c = F.lv[L - 2];
+    mmk::PStep<TV>& sa = add(mmk::PS_COARSE_A, F.Tm.n);
+    sa.A = mmk::POp<TV>{F.Tm.n, 5, F.Tm.ptr, F.Tm.col, F.Tm.val};
+    sa.x = c.b;
+    sa.y = F.tvec;
+    mmk::PStep<TV>& sb = add(mmk::PS_COARSE_B, (F.fn + 32 / mmk::CB_LANES - 1) / (32 / mmk::CB_LANES));
+    sb.A.n = F.fn;
+    while ((1 << sb.A.lg) < mmk::CB_LANES) ++sb.A.lg;
+    sb.x = F.zvec;
+    sb.b = F.tvec;
+    sb.y = c.x2;
+    a.nc = a.zr = F.fc;
+    a.M = F.W;
+  } else {
+    mmk::PStep<TV>& sd = add(mmk::PS_DENSE, F.n_coarse);
+    sd.A.n = F.n_coarse;
+    sd.A.lg = 5;
+    sd.x = F.lv[L - 1].b;
+    sd.y = F.lv[L - 1].x2;
+    a.nc = F.n_coarse;
+    a.M = F.Ainv;
+  }
+  for (int l = fused ? L - 3 : L - 2; l >= 0; --l) {
+    auto& c = F.lv[l];
+    rows(mmk::PS_PROLONG, c.P, F.lv[l + 1].x2, c.x, nullptr, c.x, nullptr);
+    if (l > 0) rows(mmk::PS_SMOOTH, c.A, c.x, c.b, c.s, c.x2, nullptr);
+  }
+  add(mmk::PS_SMOOTH0, parts).A = persistent_op(F.lv[0].A);
+  add(mmk::PS_DIR, parts);
+  add(mmk::PS_STEP, parts);
+  return blocks;
+}
+
+template <class TP, class TV>
+void launch_persistent(mm_problem* h, SolverT<TP>& S, SolverT<TV>& F, double tol, int maxiter) {
+  mmk::PcgArgs<TP, TV> a{};
+  const int blocks = persistent_args(h, S, F, a);
+  a.tol = tol;
+  a.maxiter = maxiter;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  if (a.cluster) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = blocks;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+  } else {
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+  }
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(mmk::PT);
+  const int parts = a.kshift ? (a.G * mmk::WPB) >> a.kshift : 0;  // a block folds its share of these and of b.b's
+  cfg.dynamicSmemBytes = (size_t)((std::max(parts, a.Gdot) + blocks - 1) / blocks) * BS * sizeof(double);
+  cfg.stream = h->st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  auto kern = mmk::k_pcg_persistent<TP, TV>;
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  CK(cudaLaunchKernelEx(&cfg, kern, a));
+  LAUNCH_CHECK();
+}
+
 // PCG on S.x (initial guess in, solution out) for the right-hand side S.b; stops on the recursive
 // residual r.r <= tol^2 b.b or maxiter (src/poisson_solve.py:422-478).  Returns iterations and r.r.
 // the work of a PCG solve before its loop: b.b, the scalars, r0 = b - A x0 and z0 = M^-1 r0
@@ -1028,7 +1241,7 @@ void enqueue_pcg_start(mm_problem* h, SolverT<T>& S, double tol, int maxiter) {
   const double w = sizeof(T);
   tagged<T>(h, MM_PROF_INIT_RESIDUAL, 0, mat_bytes(l0.A) + 5.0 * w * N, [&] {
     launch(h, mmk::k_init_residual<T>, grid_ilp(N), BS, l0.A.s, S.x, S.b, S.r, ml ? l0.s : nullptr, l0.x, S.sc,
-                                                             h->d_part);
+           h->d_part, red_kshift(N));
     LAUNCH_CHECK();
   });
   if (ml) enqueue_vcycle<T>(h, S, S.r, S.z, false, nullptr);
@@ -1038,9 +1251,13 @@ void enqueue_pcg_start(mm_problem* h, SolverT<T>& S, double tol, int maxiter) {
 template <class T>
 void run_pcg(mm_problem* h, SolverT<T>& S, double tol, int maxiter, int* iters, double* r2_out,
              PcgPending* pend = nullptr) {
-  enqueue_pcg_start<T>(h, S, tol, maxiter);
-  const bool graph = h->use_graph && !h->prof && loop_graph_or_retry(h, S, [&] { enqueue_iteration<T>(h, S); });
-  if (graph) {
+  const bool one = persistent_ok(h, S);
+  if (!one) enqueue_pcg_start<T>(h, S, tol, maxiter);
+  const bool graph = !one && h->use_graph && !h->prof &&
+                     loop_graph_or_retry(h, S, [&] { enqueue_iteration<T>(h, S); });
+  if (one) {
+    launch_persistent<T, T>(h, S, S, tol, maxiter);
+  } else if (graph) {
     CK(cudaGraphLaunch(S.exec, h->st));
   } else if (h->prof) {
     // profiled: read `done` after every step so that no launch runs past convergence
@@ -1088,18 +1305,20 @@ void enqueue_iteration_mp(mm_problem* h) {
   const bool df = h->a0df_ok && h->split_a0;
   if (df) {
     tagged<double>(h, MM_PROF_PCG_DIR, 0, mat_bytes(l0.A) + 4.0 * N + 4.0 * 8.0 * N, [&] {
-      launch(h, mmk::k_pcg_dir_df, grid_ilp(N), BS, h->a0df, (const float*)F.z, S.p, S.Ap, S.sc, h->d_part);
+      launch(h, mmk::k_pcg_dir_df, grid_ilp(N), BS, h->a0df, (const float*)F.z, S.p, S.Ap, S.sc, h->d_part,
+             red_kshift(N));
       LAUNCH_CHECK();
     });
   } else {
     tagged<double>(h, MM_PROF_PCG_DIR, 0, mat_bytes(l0.A) + 5.0 * 8.0 * N, [&] {
-      launch(h, mmk::k_pcg_dir<double>, grid_ilp(N), BS, l0.A.s, S.z, S.p, S.Ap, S.sc, h->d_part);
+      launch(h, mmk::k_pcg_dir<double>, grid_ilp(N), BS, l0.A.s, S.z, S.p, S.Ap, S.sc, h->d_part,
+           red_kshift(N));
       LAUNCH_CHECK();
     });
   }
   tagged<double>(h, MM_PROF_PCG_STEP, 0, 6.0 * 8.0 * N + 3.0 * 4.0 * N, [&] {
     launch(h, mmk::k_pcg_step_mp, grid_ilp(N), BS, N, S.x, S.r, S.p, S.Ap, F.lv[0].s, F.r, F.lv[0].x, S.sc,
-           h->d_part);
+           h->d_part, red_kshift(N));
     LAUNCH_CHECK();
   });
   enqueue_vcycle<float>(h, F, F.r, F.z, true, &S.sc->done, S.sc, df ? nullptr : S.z);
@@ -1116,7 +1335,7 @@ void enqueue_pcg_mp_start(mm_problem* h, double tol, int maxiter) {
   auto& l0 = S.lv[0];
   tagged<double>(h, MM_PROF_INIT_RESIDUAL, 0, mat_bytes(l0.A) + 3.0 * 8.0 * N, [&] {
     launch(h, mmk::k_init_residual<double>, grid_ilp(N), BS, l0.A.s, S.x, S.b, S.r, (const double*)nullptr,
-           l0.x, S.sc, h->d_part);
+           l0.x, S.sc, h->d_part, red_kshift(N));
     LAUNCH_CHECK();
   });
   launch(h, mmk::k_split_mp, grid_elem(N), BS, N, S.r, F.lv[0].s, F.r, F.lv[0].x);
@@ -1126,9 +1345,13 @@ void enqueue_pcg_mp_start(mm_problem* h, double tol, int maxiter) {
 
 void run_pcg_mp(mm_problem* h, double tol, int maxiter, int* iters, double* r2_out, PcgPending* pend = nullptr) {
   auto& S = h->s64;
-  enqueue_pcg_mp_start(h, tol, maxiter);
-  const bool graph = h->use_graph && !h->prof && loop_graph_or_retry(h, S, [&] { enqueue_iteration_mp(h); });
-  if (graph) {
+  const bool one = persistent_ok(h, h->s32) && h->use_a0df();
+  if (!one) enqueue_pcg_mp_start(h, tol, maxiter);
+  const bool graph = !one && h->use_graph && !h->prof &&
+                     loop_graph_or_retry(h, S, [&] { enqueue_iteration_mp(h); });
+  if (one) {
+    launch_persistent<double, float>(h, S, h->s32, tol, maxiter);
+  } else if (graph) {
     CK(cudaGraphLaunch(S.exec, h->st));
   } else {
     // host-polled: read `done` every fourth iteration (every step when profiling)
@@ -1768,17 +1991,25 @@ void enqueue_demag_nested(mm_problem* h, const double* m, double* U, double tol,
   }
   auto& S = h->s64;
   const bool mp = h->fp32_precond && h->s32.built && multilevel(h, h->s32);
-  if (mp) enqueue_pcg_mp_start(h, tol, maxiter);
-  else enqueue_pcg_start<double>(h, S, tol, maxiter);
-  mmk::k_cond_set<<<1, 32, 0, h->st>>>(hnd, 1u);  // the loop graph's default: one trip at least
-  LAUNCH_CHECK();
-  capture_nested_while(h, hnd, [&] {
-    const int64_t b0 = h->n_launch;
-    if (mp) enqueue_iteration_mp(h);
-    else enqueue_iteration<double>(h, S);
-    launch(h, mmk::k_set_cond, 1, 32, hnd, S.sc);
-    *per_trip = h->n_launch - b0 + 1;
-  });
+  if (mp && persistent_ok(h, h->s32) && h->use_a0df()) {
+    launch_persistent<double, float>(h, S, h->s32, tol, maxiter);
+    *per_trip = 1;
+  } else if (!mp && persistent_ok(h, S)) {
+    launch_persistent<double, double>(h, S, S, tol, maxiter);
+    *per_trip = 1;
+  } else {
+    if (mp) enqueue_pcg_mp_start(h, tol, maxiter);
+    else enqueue_pcg_start<double>(h, S, tol, maxiter);
+    mmk::k_cond_set<<<1, 32, 0, h->st>>>(hnd, 1u);  // the loop graph's default: one trip at least
+    LAUNCH_CHECK();
+    capture_nested_while(h, hnd, [&] {
+      const int64_t b0 = h->n_launch;
+      if (mp) enqueue_iteration_mp(h);
+      else enqueue_iteration<double>(h, S);
+      launch(h, mmk::k_set_cond, 1, 32, hnd, S.sc);
+      *per_trip = h->n_launch - b0 + 1;
+    });
+  }
   if (!h->has_mask) sub_mean(h, h->d_x);
   mmk::k_copy_vec<<<grid_vec(N), BS, 0, h->st>>>(N, h->d_x, U);
   LAUNCH_CHECK();
@@ -1842,15 +2073,18 @@ bool minimize_graph(mm_problem* h, MinCtx& c, double* m, double* U, double E0, b
       (uintptr_t)h->w_y, (uintptr_t)h->w_ys, (uintptr_t)h->w_d, (uintptr_t)h->w_dprev, (uintptr_t)h->w_mt,
       (uintptr_t)h->w_Ut, (uintptr_t)h->w_gt_trial, (uintptr_t)h->d_min_bias, (uintptr_t)pr, (uintptr_t)proj,
       (uintptr_t)fp32, (uintptr_t)ff, (uintptr_t)mp, (uintptr_t)h->pdl, (uintptr_t)h->s64.epoch,
-      (uintptr_t)h->s32.epoch, (uintptr_t)cg_maxiter, (uintptr_t)bits_of(c.phi_tol), (uintptr_t)bits_of(prm->pc_reg)};
+      (uintptr_t)h->s32.epoch, (uintptr_t)h->pcg_cap, (uintptr_t)cg_maxiter, (uintptr_t)bits_of(c.phi_tol), (uintptr_t)bits_of(prm->pc_reg)};
   mm_problem::MinGraph* mg = nullptr;
   for (auto& x : h->min_graphs)
     if (x.key == key) mg = &x;
   if (!mg) {
     mm_problem::MinGraph ng{key, nullptr, nullptr, 0, 0, 0, 0};
     bool ok = cudaGraphCreate(&ng.g, 0) == cudaSuccess;
-    cudaGraphConditionalHandle hnd[4];  // outer loop, inner solve, line search, demag PCG
-    for (int i = 0; i < 4 && ok; ++i) ok = cudaGraphConditionalHandleCreate(&hnd[i], ng.g, 0, 0) == cudaSuccess;
+    cudaGraphConditionalHandle hnd[4] = {};  // outer loop, inner solve, line search, demag PCG
+    // a handle without a node makes the graph invalid: none for the demag PCG as one launch
+    const int handles = (mp ? persistent_ok(h, h->s32) && h->use_a0df() : persistent_ok(h, h->s64)) ? 3 : 4;
+    for (int i = 0; i < handles && ok; ++i)
+      ok = cudaGraphConditionalHandleCreate(&hnd[i], ng.g, 0, 0) == cudaSuccess;
     const int64_t saved = h->n_launch;
     if (ok) ok = cudaStreamBeginCaptureToGraph(h->st, ng.g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) ==
                  cudaSuccess;
@@ -3069,6 +3303,9 @@ int mm_create(int N, int E, const int* conn, const double* volume, const double*
       CK(cudaGetDevice(&dev));
       CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
       if (sms > 0) g_vec_cap = std::min(4 * sms, MAXG);
+      int coop = 0;
+      CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+      h->coop_sms = h->pcg_cap = coop ? sms : 0;
     }
     CK(cudaEventCreate(&h->ev0));
     CK(cudaEventCreate(&h->ev1));
@@ -3132,6 +3369,7 @@ int mm_create(int N, int E, const int* conn, const double* volume, const double*
     CK(cudaMemsetAsync(h->d_part, 0, (size_t)mmk::NRED * MAXG * sizeof(double), h->st));
     h->d_sc = h->alloc<mmk::Scalars>(1);
     CK(cudaMemsetAsync(h->d_sc, 0, sizeof(mmk::Scalars), h->st));  // ticket counters start at zero
+    h->d_pbar = h->alloc<mmk::PBar>(1);
     h->d_sc32 = h->alloc<mmk::Scalars>(1);
     CK(cudaMemsetAsync(h->d_sc32, 0, sizeof(mmk::Scalars), h->st));
     h->h_sc = (mmk::Scalars*)pinned_get();
@@ -3372,6 +3610,7 @@ static cudaEvent_t upload_x0(mm_problem* h, const double* x0) {
 int mm_solve_u(mm_problem* h, const double* m, double* U, double tol, int maxiter, int* iters, double* rel_res) {
   if (!h || !m || !U || !(tol >= 0) || maxiter < 0) return MM_ERR_ARG;
   return guarded(h, [&] {
+    SolveScope in_flight(h);
     CK(cudaMemcpyAsync(h->d_m, m, 3 * (size_t)h->N * sizeof(double), cudaMemcpyHostToDevice, h->st));
     const cudaEvent_t ready = upload_x0(h, U);
     return solve_dev(h, h->d_m, h->d_U, tol, maxiter, iters, rel_res, U, ready);
@@ -3382,6 +3621,7 @@ int mm_solve_u_x0(mm_problem* h, const double* m, const double* x0, double* U_ou
                   int* iters, double* rel_res) {
   if (!h || !m || !x0 || !U_out || !(tol >= 0) || maxiter < 0) return MM_ERR_ARG;
   return guarded(h, [&] {
+    SolveScope in_flight(h);
     CK(cudaMemcpyAsync(h->d_m, m, 3 * (size_t)h->N * sizeof(double), cudaMemcpyHostToDevice, h->st));
     const cudaEvent_t ready = upload_x0(h, x0);
     return solve_dev(h, h->d_m, h->d_U, tol, maxiter, iters, rel_res, U_out, ready);
@@ -3391,7 +3631,10 @@ int mm_solve_u_x0(mm_problem* h, const double* m, const double* x0, double* U_ou
 int mm_solve_u_dev(mm_problem* h, const double* d_m, double* d_U, double tol, int maxiter, int* iters,
                    double* rel_res) {
   if (!h || !d_m || !d_U || !(tol >= 0) || maxiter < 0) return MM_ERR_ARG;
-  return guarded(h, [&] { return solve_dev(h, d_m, d_U, tol, maxiter, iters, rel_res); });
+  return guarded(h, [&] {
+    SolveScope in_flight(h);
+    return solve_dev(h, d_m, d_U, tol, maxiter, iters, rel_res);
+  });
 }
 
 int mm_set_magnetoelastic(mm_problem* h, int n, const double* k1me, const double* k1me_p) {
@@ -3494,6 +3737,7 @@ int mm_minimize(mm_problem* h, const double* B, double* m, double* U, const mm_m
   if (prm->method < 0 || prm->method >= MM_METHOD_COUNT || prm->max_iter < 0) return MM_ERR_ARG;
   return guarded(h, [&] {
     if (!h->poisson_built) throw Fail{MM_ERR_STATE, "mm_build_poisson must be called first"};
+    SolveScope in_flight(h);
     const size_t n3 = 3 * (size_t)h->N;
     // the minimizer owns d_m / d_U as its state buffers; they may be swapped with its trial buffers
     CK(cudaMemcpyAsync(h->d_m, m, n3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
@@ -3517,6 +3761,7 @@ int mm_minimize_dev(mm_problem* h, const double* B, double* d_m, double* d_U, co
   if (prm->method < 0 || prm->method >= MM_METHOD_COUNT || prm->max_iter < 0) return MM_ERR_ARG;
   return guarded(h, [&] {
     if (!h->poisson_built) throw Fail{MM_ERR_STATE, "mm_build_poisson must be called first"};
+    SolveScope in_flight(h);
     const size_t n3 = 3 * (size_t)h->N;
     // the minimizer swaps its state with its trial buffers, so it runs on the problem's own buffers;
     // the caller's arrays are copied in and out on the device
@@ -3554,7 +3799,7 @@ int mm_time_kernel(mm_problem* h, int kernel, int reps, double* ms, double* byte
       } else if (kernel == MM_KERNEL_SMOOTH) {
         const double* s = l0->s ? l0->s : h->d_U;
         launch(h, mmk::k_smooth_dot<double>, grid_ilp(l0->n), BS, l0->A.s, h->d_U, h->d_b, s, h->d_out, h->d_sc, h->d_part,
-                                                                nullptr, (double*)nullptr);
+                                                                nullptr, (double*)nullptr, red_kshift(N));
         LAUNCH_CHECK();
       } else if (kernel == MM_KERNEL_ENERGY) {
         const double B[3] = {0.0, 0.0, 1.0};
@@ -3629,9 +3874,37 @@ float time_ms(mm_problem* h, int reps, const std::function<void()>& f) {
   return ms / reps;
 }
 
+// Time of V-cycles of solver S: four PCG iterations as one launch where its solves run so (a constant right-hand
+// side and no tolerance; per V-cycle), else V-cycles back to back.
+template <class T>
+float vcycle_ms(mm_problem* h, SolverT<T>& S, int reps) {
+  const bool mp = h->fp32_precond && std::is_same<T, float>::value;
+  const bool solves = std::is_same<T, float>::value ? (h->mixed || mp) : !(h->mixed || h->fp32_precond);
+  if (!solves || !persistent_ok(h, S) || (mp && !h->use_a0df()))
+    return time_ms<T>(h, reps, [&] { enqueue_precond<T>(h, S, S.r, S.z); });
+  SolverT<double>& D = h->s64;
+  const size_t bytes = (size_t)h->N * (mp ? sizeof(double) : sizeof(T));
+  void* b = mp ? (void*)D.b : (void*)S.b;
+  void* x = mp ? (void*)D.x : (void*)S.x;
+  CK(cudaMemsetAsync(b, 0x3f, bytes, h->st));
+  CK(cudaMemsetAsync(x, 0, bytes, h->st));
+  constexpr int ITERS = 4;
+  const float ms = time_ms<T>(h, reps, [&] {
+    if constexpr (std::is_same<T, float>::value) {
+      if (mp) launch_persistent<double, float>(h, D, S, 0.0, ITERS);
+      else launch_persistent<float, float>(h, S, S, 0.0, ITERS);
+    } else {
+      launch_persistent<T, T>(h, S, S, 0.0, ITERS);
+    }
+  });
+  CK(cudaMemsetAsync(b, 0, bytes, h->st));  // D m writes the magnetic rows only
+  CK(cudaMemsetAsync(x, 0, bytes, h->st));
+  return ms / ITERS;
+}
+
 // Lanes per row of one compressed-row operator: every candidate is timed in context, as the time of
-// whole V-cycles (back to back, so cache state and neighbouring kernels are those of a solve; an
-// operator timed alone, L2-hot, prefers fewer lanes than it should), and the fastest is kept.
+// whole V-cycles or PCG iterations (cache state and neighbours are those of a solve; an operator timed
+// alone, L2-hot, prefers fewer lanes than it should), and the fastest is kept.
 template <class T>
 void tune_csr(mm_problem* h, SolverT<T>& S, DevMatT<T>& M, const mm::HostCSR& host, int reps, const char* tag,
               int level, std::string& rep) {
@@ -3643,7 +3916,7 @@ void tune_csr(mm_problem* h, SolverT<T>& S, DevMatT<T>& M, const mm::HostCSR& ho
   std::string times;
   for (int t : {1, 2, 4, 8, 16, 32}) {
     M.tpr = t;
-    const float ms = time_ms<T>(h, reps, [&] { enqueue_precond<T>(h, S, S.r, S.z); });
+    const float ms = vcycle_ms<T>(h, S, reps);
     times += (times.empty() ? "" : ",") + std::to_string(1e3 * ms);
     if (t == before) before_ms = ms;
     if (ms < best_ms) {
@@ -3684,7 +3957,7 @@ std::string tune_fuse_restrict(mm_problem* h, SolverT<T>& S, int bit, int reps) 
   float ms[2];
   for (int on = 0; on < 2; ++on) {
     h->fuse_restrict = on ? (saved | (1 << bit)) : (saved & ~(1 << bit));
-    ms[on] = time_ms<T>(h, reps, [&] { enqueue_precond<T>(h, S, S.r, S.z); });
+    ms[on] = vcycle_ms<T>(h, S, reps);
   }
   h->fuse_restrict = ms[1] < ms[0] ? (saved | (1 << bit)) : (saved & ~(1 << bit));
   drop_graph(S);
@@ -3695,13 +3968,11 @@ std::string tune_fuse_restrict(mm_problem* h, SolverT<T>& S, int bit, int reps) 
 template <class T>
 std::string tune_fuse(mm_problem* h, SolverT<T>& S, int bit, int reps) {
   if (!S.built || !S.fused || !multilevel(h, S)) return "null";
-  T* r = S.r;
-  T* z = S.z;
   const int saved = h->coarse_fuse;
   float ms[2];
   for (int on = 0; on < 2; ++on) {
     h->coarse_fuse = on ? (saved | (1 << bit)) : (saved & ~(1 << bit));
-    ms[on] = time_ms<T>(h, reps, [&] { enqueue_precond<T>(h, S, r, z); });
+    ms[on] = vcycle_ms<T>(h, S, reps);
   }
   h->coarse_fuse = ms[1] < ms[0] ? (saved | (1 << bit)) : (saved & ~(1 << bit));
   drop_graph(S);

@@ -131,6 +131,11 @@ __device__ __forceinline__ void grid_reduce(double v0, double v1, Scalars* sc, d
 // Thread 0 publishes the block's partials and takes a ticket with one acquire-release atomic (its
 // release orders the partials before the ticket); the block holding the last ticket loads every
 // partial at once (independent, unrolled loads), sums them in block order and runs the follow-up.
+// The final sum over `G` partials (slot0, and slot1 unless < 0) and its follow-up, by one whole block.
+template <bool MAX>
+__device__ __forceinline__ void grid_total(int G, Scalars* sc, const double* part, int slot0, int slot1, int post,
+                                           double post_arg);
+
 template <bool MAX>
 __device__ __forceinline__ void grid_finish(double v0, double v1, Scalars* sc, double* part, int slot0, int slot1,
                                             int post, double post_arg) {
@@ -143,66 +148,69 @@ __device__ __forceinline__ void grid_finish(double v0, double v1, Scalars* sc, d
     s_last = (t == gridDim.x - 1) ? 1u : 0u;
   }
   __syncthreads();
-  if (s_last) {
-    __threadfence();
-    const int G = (int)gridDim.x;
-    const double* pa = part + (size_t)slot0 * MAXG;
-    const double* pb = part + (size_t)(slot1 >= 0 ? slot1 : slot0) * MAXG;
-    double a = 0.0, b = 0.0;
+  if (s_last) grid_total<MAX>((int)gridDim.x, sc, part, slot0, slot1, post, post_arg);
+}
+
+template <bool MAX>
+__device__ __forceinline__ void grid_total(int G, Scalars* sc, const double* part, int slot0, int slot1, int post,
+                                           double post_arg) {
+  __threadfence();
+  const double* pa = part + (size_t)slot0 * MAXG;
+  const double* pb = part + (size_t)(slot1 >= 0 ? slot1 : slot0) * MAXG;
+  double a = 0.0, b = 0.0;
 #pragma unroll
-    for (int k = 0; k < MAXG / BS; ++k) {
-      const int i = threadIdx.x + k * BS;
-      if (i < G) {
-        const double xa = __ldcg(pa + i);
-        a = MAX ? fmax(a, xa) : a + xa;
-        if (slot1 >= 0) {
-          const double xb = __ldcg(pb + i);
-          b = MAX ? fmax(b, xb) : b + xb;
-        }
+  for (int k = 0; k < MAXG / BS; ++k) {
+    const int i = threadIdx.x + k * BS;
+    if (i < G) {
+      const double xa = __ldcg(pa + i);
+      a = MAX ? fmax(a, xa) : a + xa;
+      if (slot1 >= 0) {
+        const double xb = __ldcg(pb + i);
+        b = MAX ? fmax(b, xb) : b + xb;
       }
     }
-    a = block_reduce<MAX>(a);
-    if (slot1 >= 0) b = block_reduce<MAX>(b);
-    if (threadIdx.x == 0) {
-      sc->red[slot0] = a;
-      if (slot1 >= 0) sc->red[slot1] = b;
-      sc->cnt[slot0] = 0u;
-      if (post == POST_PAP) {
-        sc->alpha = sc->rz / (a + 1e-30);
-        sc->alpha_f = (float)sc->alpha;
-      } else if (post == POST_R2_STEP || post == POST_R2_INIT) {
-        if (post == POST_R2_STEP) sc->it += 1;
-        if (a <= sc->tol2 || sc->it >= sc->maxiter) sc->done = 1;
-      } else if (post == POST_RZ) {
-        sc->beta = sc->rz_valid ? a / (sc->rz + 1e-30) : 0.0;
-        sc->beta_f = (float)sc->beta;
-        sc->rz = a;
-        sc->rz_valid = 1;
-      } else if (post == POST_MEAN) {
-        sc->red[slot0] = a / post_arg;
-      } else if (post == POST_IN_INIT) {
-        sc->in_rho = a;
-        sc->in_target = sc->in_tol2 * a;
-        sc->in_done = !(sc->in_it < sc->in_max && a > sc->in_target && a > 1e-25 && a < 1e20);
-      } else if (post == POST_IN_PAP) {
-        const double alpha = sc->in_rho / (a + 1e-30);
-        const double dq = 0.5 * alpha * sc->in_rho;
-        const bool stag = (sc->in_it > 0) && (dq <= sc->in_nu * sc->in_Q);
-        sc->in_alpha = alpha;
-        sc->in_alpha_f = (float)alpha;
-        sc->in_dq = dq;
-        sc->in_stop = (a <= 0.0) || stag;
-      } else if (post == POST_IN_RHO) {
-        const double rho = a;
-        sc->in_beta = rho / (sc->in_rho + 1e-30);
-        sc->in_beta_f = (float)sc->in_beta;
-        sc->in_rho = rho;
-        sc->in_Q = sc->in_Q + sc->in_dq;
-        sc->in_it += (sc->in_cpp && sc->in_stop) ? 0 : 1;
-        sc->red[R_D] = (double)sc->in_it;  // read by the host with the fallback test's sums
-        sc->in_done = sc->in_stop ||
-                      !(sc->in_it < sc->in_max && rho > sc->in_target && rho > 1e-25 && rho < 1e20);
-      }
+  }
+  a = block_reduce<MAX>(a);
+  if (slot1 >= 0) b = block_reduce<MAX>(b);
+  if (threadIdx.x == 0) {
+    sc->red[slot0] = a;
+    if (slot1 >= 0) sc->red[slot1] = b;
+    sc->cnt[slot0] = 0u;
+    if (post == POST_PAP) {
+      sc->alpha = sc->rz / (a + 1e-30);
+      sc->alpha_f = (float)sc->alpha;
+    } else if (post == POST_R2_STEP || post == POST_R2_INIT) {
+      if (post == POST_R2_STEP) sc->it += 1;
+      if (a <= sc->tol2 || sc->it >= sc->maxiter) sc->done = 1;
+    } else if (post == POST_RZ) {
+      sc->beta = sc->rz_valid ? a / (sc->rz + 1e-30) : 0.0;
+      sc->beta_f = (float)sc->beta;
+      sc->rz = a;
+      sc->rz_valid = 1;
+    } else if (post == POST_MEAN) {
+      sc->red[slot0] = a / post_arg;
+    } else if (post == POST_IN_INIT) {
+      sc->in_rho = a;
+      sc->in_target = sc->in_tol2 * a;
+      sc->in_done = !(sc->in_it < sc->in_max && a > sc->in_target && a > 1e-25 && a < 1e20);
+    } else if (post == POST_IN_PAP) {
+      const double alpha = sc->in_rho / (a + 1e-30);
+      const double dq = 0.5 * alpha * sc->in_rho;
+      const bool stag = (sc->in_it > 0) && (dq <= sc->in_nu * sc->in_Q);
+      sc->in_alpha = alpha;
+      sc->in_alpha_f = (float)alpha;
+      sc->in_dq = dq;
+      sc->in_stop = (a <= 0.0) || stag;
+    } else if (post == POST_IN_RHO) {
+      const double rho = a;
+      sc->in_beta = rho / (sc->in_rho + 1e-30);
+      sc->in_beta_f = (float)sc->in_beta;
+      sc->in_rho = rho;
+      sc->in_Q = sc->in_Q + sc->in_dq;
+      sc->in_it += (sc->in_cpp && sc->in_stop) ? 0 : 1;
+      sc->red[R_D] = (double)sc->in_it;  // read by the host with the fallback test's sums
+      sc->in_done = sc->in_stop ||
+                    !(sc->in_it < sc->in_max && rho > sc->in_target && rho > 1e-25 && rho < 1e20);
     }
   }
 }
@@ -291,6 +299,44 @@ __device__ __forceinline__ double block_total(Acc<T>& acc) {
     __syncthreads();
     return s_out;
   }
+}
+
+// Grid reduction of the kernels that take ROW_LOOP's rows: one partial per chunk of 1 << kshift warps
+// (8 warps: the block's; 1: a warp's), chunk totals in `part` in row order.  Small problems take chunks of
+// one warp (red_kshift): the one-launch PCG (mm_pcg.cuh), whose reductions are these, then spreads them over
+// every SM, each of which does two FP64 operations a clock.
+template <class T>
+__device__ __forceinline__ void chunk_finish(Acc<T>& acc, Scalars* sc, double* part, int slot, int post, int kshift) {
+  __shared__ double s_v[BS];
+  __shared__ unsigned s_last;
+  constexpr int W = BS / 32;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int k = 1 << kshift, per = W >> kshift;  // warps of a chunk, chunks of a block
+  double v = 0.0;
+  if constexpr (std::is_same<T, double>::value) v = acc.s;
+  else v = acc.warp_total();  // lane 0
+  __syncthreads();
+  s_v[threadIdx.x] = v;
+  __syncthreads();
+  if (wid < per) {
+    double t;
+    if constexpr (std::is_same<T, double>::value) {
+      t = s_v[32 * (wid << kshift) + lane];
+      for (int j = 1; j < k; ++j) t += s_v[32 * ((wid << kshift) + j) + lane];
+      t = warp_sum(t);
+    } else {
+      t = 0.0;
+      for (int j = 0; j < k; ++j) t += s_v[32 * ((wid << kshift) + j)];
+    }
+    if (lane == 0) part[(size_t)slot * MAXG + blockIdx.x * per + wid] = t;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    cuda::atomic_ref<unsigned, cuda::thread_scope_device> ticket(sc->cnt[slot]);
+    s_last = (ticket.fetch_add(1u, cuda::memory_order_acq_rel) == gridDim.x - 1) ? 1u : 0u;
+  }
+  __syncthreads();
+  if (s_last) grid_total<false>((int)gridDim.x * per, sc, part, slot, -1, post, 0.0);
 }
 
 // Sliced ELL, slice height 32, entries paired: entry k of row r lives at
@@ -518,7 +564,7 @@ __global__ void __launch_bounds__(BS) k_sell(SellT<T> A, const T* __restrict__ x
 template <class T>
 __global__ void __launch_bounds__(BS) k_init_residual(SellT<T> A, const T* __restrict__ x, const T* __restrict__ b,
                                                       T* __restrict__ r, const T* __restrict__ s, T* __restrict__ xv,
-                                                      Scalars* sc, double* part) {
+                                                      Scalars* sc, double* part, int kshift) {
   pdl_entry();
   Acc<T> acc;
   ROW_LOOP(A.n) {
@@ -536,7 +582,7 @@ __global__ void __launch_bounds__(BS) k_init_residual(SellT<T> A, const T* __res
       if (s) xv[i] = s[i] * ri;
     }
   }
-  grid_finish(block_total(acc), 0.0, sc, part, R_R2, -1, POST_R2_INIT);
+  chunk_finish(acc, sc, part, R_R2, POST_R2_INIT, kshift);
 }
 
 // PCG direction update fused with the operator product:
@@ -544,7 +590,7 @@ __global__ void __launch_bounds__(BS) k_init_residual(SellT<T> A, const T* __res
 // (A p_new = A z + beta A p_old, so the product is taken on z, complete before the launch)
 template <class T>
 __global__ void __launch_bounds__(BS) k_pcg_dir(SellT<T> A, const T* __restrict__ z, T* __restrict__ p,
-                                                T* __restrict__ Ap, Scalars* sc, double* part) {
+                                                T* __restrict__ Ap, Scalars* sc, double* part, int kshift) {
   pdl_entry();
   if (sc->done) return;
   const T beta = scal<T>(sc->beta, sc->beta_f);
@@ -566,7 +612,7 @@ __global__ void __launch_bounds__(BS) k_pcg_dir(SellT<T> A, const T* __restrict_
       acc.add(pn, apn);
     }
   }
-  grid_finish(block_total(acc), 0.0, sc, part, R_PAP, -1, POST_PAP);
+  chunk_finish(acc, sc, part, R_PAP, POST_PAP, kshift);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -649,7 +695,8 @@ __device__ __forceinline__ void sell_rows_df(const SellDF& A, const float* __res
 // A z is taken with the split operator (FP32 pipes) and only the per-row updates run in FP64:
 //   p = z + beta p ; Ap = A z + beta Ap ; p.Ap -> red[R_PAP]
 __global__ void __launch_bounds__(BS) k_pcg_dir_df(SellDF A, const float* __restrict__ z, double* __restrict__ p,
-                                                   double* __restrict__ Ap, Scalars* sc, double* part) {
+                                                   double* __restrict__ Ap, Scalars* sc, double* part,
+                                                   int kshift) {
   pdl_entry();
   if (sc->done) return;
   const double beta = sc->beta;
@@ -672,14 +719,14 @@ __global__ void __launch_bounds__(BS) k_pcg_dir_df(SellDF A, const float* __rest
       acc.add(pn, apn);
     }
   }
-  grid_finish(block_total(acc), 0.0, sc, part, R_PAP, -1, POST_PAP);
+  chunk_finish(acc, sc, part, R_PAP, POST_PAP, kshift);
 }
 
 // x += alpha p ; r -= alpha Ap ; r.r -> red[R_R2] ; xv = s .* r
 template <class T>
 __global__ void __launch_bounds__(BS) k_pcg_step(int n, T* __restrict__ x, T* __restrict__ r, const T* __restrict__ p,
                                                  const T* __restrict__ Ap, const T* __restrict__ s0, T* __restrict__ xv,
-                                                 Scalars* sc, double* part) {
+                                                 Scalars* sc, double* part, int kshift) {
   pdl_entry();
   if (sc->done) return;
   const T alpha = scal<T>(sc->alpha, sc->alpha_f);
@@ -698,7 +745,7 @@ __global__ void __launch_bounds__(BS) k_pcg_step(int n, T* __restrict__ x, T* __
       if (s0) xv[i] = s0[i] * ri;
     }
   }
-  grid_finish(block_total(acc), 0.0, sc, part, R_R2, -1, POST_R2_STEP);
+  chunk_finish(acc, sc, part, R_R2, POST_R2_STEP, kshift);
 }
 
 // FP64 PCG preconditioned by the FP32 V-cycle: x += alpha p ; r -= alpha Ap (FP64) ; r.r -> red[R_R2] ;
@@ -706,7 +753,8 @@ __global__ void __launch_bounds__(BS) k_pcg_step(int n, T* __restrict__ x, T* __
 __global__ void __launch_bounds__(BS) k_pcg_step_mp(int n, double* __restrict__ x, double* __restrict__ r,
                                                     const double* __restrict__ p, const double* __restrict__ Ap,
                                                     const float* __restrict__ s0, float* __restrict__ r32,
-                                                    float* __restrict__ xv, Scalars* sc, double* part) {
+                                                    float* __restrict__ xv, Scalars* sc, double* part,
+                                                    int kshift) {
   pdl_entry();
   if (sc->done) return;
   const double alpha = sc->alpha;
@@ -727,7 +775,7 @@ __global__ void __launch_bounds__(BS) k_pcg_step_mp(int n, double* __restrict__ 
       xv[i] = s0[i] * rf;
     }
   }
-  grid_finish(block_total(acc), 0.0, sc, part, R_R2, -1, POST_R2_STEP);
+  chunk_finish(acc, sc, part, R_R2, POST_R2_STEP, kshift);
 }
 
 // r32 = fl32(r), xv = s0 .* r32 (before the first V-cycle of a solve)
@@ -984,7 +1032,7 @@ template <class T>
 __global__ void __launch_bounds__(BS) k_smooth_dot(SellT<T> A, const T* __restrict__ x, const T* __restrict__ b,
                                                    const T* __restrict__ s, T* __restrict__ y, Scalars* sc,
                                                    double* part, const int* __restrict__ done,
-                                                   double* __restrict__ y64) {
+                                                   double* __restrict__ y64, int kshift) {
   pdl_entry();
   if (done && *done) return;
   Acc<T> acc;
@@ -1003,7 +1051,7 @@ __global__ void __launch_bounds__(BS) k_smooth_dot(SellT<T> A, const T* __restri
       acc.add(b[i], yi);
     }
   }
-  if (part) grid_finish(block_total(acc), 0.0, sc, part, R_RZ, -1, POST_RZ);
+  if (part) chunk_finish(acc, sc, part, R_RZ, POST_RZ, kshift);
 }
 
 // condition of the graph's WHILE node: keep looping until done (bounded by maxiter + 2 trips)
