@@ -91,6 +91,17 @@ __device__ __forceinline__ double warp_max(double v) {
 // folds the block's 256 values eight to a lane, then one shuffle tree, i.e. 12 warp-wide FP64
 // instructions per block instead of a tree in every warp (48); a warp-wide FP64 add holds the SM's
 // FP64 pipe for 16 cycles on this part, so the trees were a visible share of the FP64 kernels.
+// The fold is pairwise, three adds deep instead of seven: an FP64 add takes 76 clocks, and what waits for the
+// reduction waits for its chain (the one-launch PCG of 1.3k rows 316 -> 305 us with it).
+template <bool MAX>
+__device__ __forceinline__ double fold2(double a, double b) {
+  return MAX ? fmax(a, b) : a + b;
+}
+template <bool MAX>
+__device__ __forceinline__ double fold8(const double (&u)[8]) {
+  return fold2<MAX>(fold2<MAX>(fold2<MAX>(u[0], u[1]), fold2<MAX>(u[2], u[3])),
+                    fold2<MAX>(fold2<MAX>(u[4], u[5]), fold2<MAX>(u[6], u[7])));
+}
 template <bool MAX>
 __device__ __forceinline__ double block_reduce(double v) {
   __shared__ double s_red[BS];
@@ -99,12 +110,11 @@ __device__ __forceinline__ double block_reduce(double v) {
   s_red[threadIdx.x] = v;
   __syncthreads();
   if (threadIdx.x < 32) {
-    double t = s_red[threadIdx.x];
+    static_assert(BS == 256, "eight values a lane");
+    double u[8];
 #pragma unroll
-    for (int k = 1; k < BS / 32; ++k) {
-      const double u = s_red[threadIdx.x + 32 * k];
-      t = MAX ? fmax(t, u) : t + u;
-    }
+    for (int k = 0; k < 8; ++k) u[k] = s_red[threadIdx.x + 32 * k];
+    double t = fold8<MAX>(u);
     t = MAX ? warp_max(t) : warp_sum(t);
     if (threadIdx.x == 0) s_out = t;
   }
@@ -302,7 +312,7 @@ __device__ __forceinline__ double block_total(Acc<T>& acc) {
 }
 
 // Grid reduction of the kernels that take ROW_LOOP's rows: one partial per chunk of 1 << kshift warps
-// (8 warps: the block's; 1: a warp's), chunk totals in `part` in row order.  Small problems take chunks of
+// (kshift 3: the block's; 0: a warp's), chunk totals in `part` in row order.  Small problems take chunks of
 // one warp (red_kshift): the one-launch PCG (mm_pcg.cuh), whose reductions are these, then spreads them over
 // every SM, each of which does two FP64 operations a clock.
 template <class T>
@@ -322,7 +332,12 @@ __device__ __forceinline__ void chunk_finish(Acc<T>& acc, Scalars* sc, double* p
     double t;
     if constexpr (std::is_same<T, double>::value) {
       t = s_v[32 * (wid << kshift) + lane];
-      for (int j = 1; j < k; ++j) t += s_v[32 * ((wid << kshift) + j) + lane];
+      if (kshift) {
+        double u[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) u[j] = s_v[32 * (8 * wid + j) + lane];
+        t = fold8<false>(u);
+      }
       t = warp_sum(t);
     } else {
       t = 0.0;

@@ -233,30 +233,47 @@ __device__ __forceinline__ void psell2_df(const SellDF& A, const float* z, int r
   }
 }
 
+// FP64 products leave by branches on a count that the whole warp shares, since a predicated-off FP64 operation
+// still holds the FP64 pipe for its 16 clocks, eight of them for the two or three entries of a prolongation's
+// lane (lanes without an entry add zero to their sum): 59k rows' prolongation 10.6k -> 8.7k clocks, their whole
+// solve 787 -> 750 us.  FP32 products stay predicated (by branches their solves are 1-2 % slower).
 template <class T>
 __device__ __forceinline__ T pcsr_row(const int* __restrict__ ptr, const int* __restrict__ col,
                                       const T* __restrict__ val, const T* x, int row, bool valid, int lane, int lg) {
   constexpr int U = 8;
   const int tpr = 1 << lg;
   T acc = T(0);
+  int k0 = 0, e = 0;
   if (valid) {
-    const int s = __ldg(ptr + row), e = __ldg(ptr + row + 1);
+    k0 = __ldg(ptr + row) + lane;
+    e = __ldg(ptr + row + 1);
+  }
+  int left = __reduce_max_sync(0xffffffffu, e > k0 ? (e - k0 + tpr - 1) >> lg : 0);
 #pragma unroll 1
-    for (int k = s + lane; k < e; k += U * tpr) {
-      int c[U] = {};  // defined on every path: a register that only predicated loads write stays live
-      T v[U] = {}, g[U] = {};  // through the whole kernel
+  for (; left > 0; left -= U, k0 += U * tpr) {
+    int c[U] = {};  // defined on every path: a register that only predicated loads write stays live
+    T v[U] = {}, g[U] = {};  // through the whole kernel
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k0 + u * tpr < e) {
+        c[u] = __ldg(col + k0 + u * tpr);
+        v[u] = __ldg(val + k0 + u * tpr);
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k0 + u * tpr < e) g[u] = x[c[u]];
+    if constexpr (sizeof(T) == 8) {
+      do {
+#define PMADD(K)         \
+  if (K >= left) break; \
+  acc = fmaT<T>(v[K], g[K], acc);
+        PMADD(0) PMADD(1) PMADD(2) PMADD(3) PMADD(4) PMADD(5) PMADD(6) PMADD(7)
+#undef PMADD
+      } while (false);
+    } else {
 #pragma unroll
       for (int u = 0; u < U; ++u)
-        if (k + u * tpr < e) {
-          c[u] = __ldg(col + k + u * tpr);
-          v[u] = __ldg(val + k + u * tpr);
-        }
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (k + u * tpr < e) g[u] = x[c[u]];
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (k + u * tpr < e) acc = fmaT<T>(v[u], g[u], acc);
+        if (k0 + u * tpr < e) acc = fmaT<T>(v[u], g[u], acc);
     }
   }
 #pragma unroll 1
@@ -348,10 +365,10 @@ __device__ __noinline__ void ptotal(PScal& ps, const double* part, int slot, int
     return;
   }
   asm volatile("barrier.sync %0, %1;" ::"r"(bar), "n"(BS) : "memory");
-  a = s_red[tid];
+  double u[8];
 #pragma unroll
-  for (int k = 1; k < WPB; ++k) a += s_red[tid + 32 * k];
-  a = warp_sum(a);
+  for (int k = 0; k < 8; ++k) u[k] = s_red[tid + 32 * k];
+  a = warp_sum(fold8<false>(u));
   if (tid == 0) {
     if (slot == R_BB) {
       ps.bb = a;
@@ -483,19 +500,18 @@ __device__ __forceinline__ void preduce(const PcgArgs<TP, TV>& a, int kind, PSca
   meet();
   if (kshift == 0) return;
   __syncthreads();
-  const int k = 1 << kshift;
 #pragma unroll 1
   for (int c = wid; c < nc; c += PW) {
     double t;
     if constexpr (std::is_same<T, double>::value) {
-      t = s_unit[32 * (c << kshift) + lane];
-#pragma unroll 1
-      for (int j = 1; j < k; ++j) t += s_unit[32 * ((c << kshift) + j) + lane];
-      t = warp_sum(t);
+      double u[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) u[j] = s_unit[32 * (8 * c + j) + lane];
+      t = warp_sum(fold8<false>(u));
     } else {
       t = 0.0;
 #pragma unroll 1
-      for (int j = 0; j < k; ++j) t += s_unit[(c << kshift) + j];
+      for (int j = 0; j < WPB; ++j) t += s_unit[WPB * c + j];
     }
     if (lane == 0) pa[c] = t;
   }
@@ -531,10 +547,10 @@ __device__ __forceinline__ void pdot_bb(const PcgArgs<TP, TV>& a) {
   for (int c = wid; c < nc; c += PW) {
     double t;
     if constexpr (std::is_same<TP, double>::value) {
-      t = s_unit[32 * (c * WPB) + lane];
-#pragma unroll 1
-      for (int j = 1; j < WPB; ++j) t += s_unit[32 * (c * WPB + j) + lane];
-      t = warp_sum(t);
+      double u[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) u[j] = s_unit[32 * (8 * c + j) + lane];
+      t = warp_sum(fold8<false>(u));
     } else {
       t = 0.0;
 #pragma unroll 1
@@ -564,10 +580,10 @@ __device__ __forceinline__ void pcoarse_a(const PcgArgs<TP, TV>& a, const PStep<
       s_red[tb] = acc;
       asm volatile("barrier.sync 1, %0;" ::"n"(BS) : "memory");
       if (tb < 32) {
-        acc = s_red[tb];
+        double u[8];
 #pragma unroll
-        for (int k = 1; k < WPB; ++k) acc += s_red[tb + 32 * k];
-        acc = warp_sum(acc);
+        for (int k = 0; k < 8; ++k) u[k] = s_red[tb + 32 * k];
+        acc = warp_sum(fold8<false>(u));
         if (tb == 0) a.zvec[r] = (TV)acc;
       }
       asm volatile("barrier.sync 1, %0;" ::"n"(BS) : "memory");
