@@ -86,6 +86,7 @@ template <class T>
 struct DevMatT {
   mmk::SellT<T> s{};
   mmk::CsrT<T> c{};
+  mmk::SellT<T> lanes[5]{};  // the rows dealt out over 2, 4 .. 32 lanes, for the one-launch PCG (upload_lanes)
   int tpr = 1;
   int64_t nnz = 0;     // stored non-zeros (without padding)
   int64_t stored = 0;  // entries including padding
@@ -122,6 +123,7 @@ struct SolverT {
   // fused coarse correction of levels L-2 .. L-1 (x2 = T b + W (Z b)), when eligible
   bool fused = false;
   mmk::CsrT<T> Tm{};
+  mmk::SellT<T> Tml{};  // T's rows over 32 lanes (upload_lanes)
   T *W = nullptr, *Z = nullptr, *tvec = nullptr, *zvec = nullptr;
   int fn = 0, fc = 0;
   int64_t Tm_nnz = 0;
@@ -140,17 +142,19 @@ bool one_launch_rows(int64_t n) {
   return sizeof(T) == 8 || n <= 786432;
 }
 
-// Layout choice for an operator of an n-row problem: one thread per row from 64Ki rows on, else t lanes per row
-// (2..32) by the cost of a phase of the one-launch PCG on an SM in clocks: its warp instructions (an FP64 one
-// holds the SM's FP64 pipe for 16 clocks, so a row's log2 t reduction steps cost as much as its entries: 32
-// lanes on the 62-entry rows of the 40 nm cube's level-0 fused restriction spend 7 a row, 4 lanes 2.25) against
-// the latency of its dependent loads (~1400 clocks for each eight entries of a lane), which overlap in part.
-// FP32 V-cycle, a solve with it and with lanes for ~256Ki threads: 40 nm cube 700 and 799 us, 80 nm cube 1.68 and
-// 1.79 ms.  The separate kernels of larger FP32 problems want the latter.
+// Layout choice for an operator of an n-row problem.  From 64Ki rows on one thread per row, or two lanes for FP64
+// rows of 16 entries or more (two lanes' gathers share sectors, one thread's hit a row each; 1,601,613 rows, a solve
+// with 1, 2, 4 and 8 lanes: 6.13, 5.99, 6.17 and 6.66 ms).  Below, t lanes per row (2..32) by the cost of a phase of
+// the one-launch PCG on an SM in clocks: its warp instructions (an FP64 one holds the SM's FP64 pipe for 16 clocks,
+// so a row's log2 t reduction steps cost as much as its entries: 32 lanes on the 62-entry rows of the 40 nm cube's
+// level-0 fused restriction spend 7 a row, 4 lanes 2.25) against the latency of its dependent loads (~1400 clocks
+// for each eight entries of a lane), which overlap in part.  FP64 solves of the 40 nm and 80 nm cubes with these
+// lanes, half and twice as many: 726, 776 and 737 us, 1.85, 1.96 and 1.90 ms.  The separate kernels of larger FP32
+// problems want lanes for ~256Ki threads.
 template <class T>
 int choose_tpr(int64_t rows, int64_t nnz, int64_t n) {
-  if (rows >= 65536) return 1;
   const double avg = rows > 0 ? (double)nnz / (double)rows : 1.0;
+  if (rows >= 65536) return sizeof(T) == 8 && avg >= 16.0 ? 2 : 1;
   if (!one_launch_rows<T>(n)) {
     int t = 2;
     while (t < 32 && (rows * t < 262144) && t < avg) t *= 2;
@@ -568,10 +572,45 @@ struct mm_problem {
       d.c.val = upload_as<T>(A.val);
       d.stored = A.nnz();
       d.s.n = A.n_rows;
+      upload_lanes<T>(A, d);
       return d;
     }
     upload_sell<T>(A, d);
     return d;
+  }
+  // What the one-launch PCG reads of an operator with tpr > 1: its rows dealt out over tpr lanes (entry k to lane
+  // k % tpr) and the lanes laid out as the rows of a sliced ELL, so that a warp's loads of columns and values are
+  // contiguous.  Read from the compressed rows, 16 rows by two lanes each are 16 separate pieces to a load, and the
+  // L1's wavefronts took half of a restriction's time.  FP64 solves from compressed and from dealt-out rows:
+  // 59,319 rows 750 and 726 us, 357,911 rows 1913 and 1848 us (FP32 V-cycle 1674 and 1637).
+  template <class T>
+  void upload_lanes(const mm::HostCSR& A, DevMatT<T>& d) {
+    if (d.tpr == 1 || !one_launch_rows<T>(N)) return;
+    const int t = d.tpr, per = 32 / t, ns = (A.n_rows + per - 1) / per;
+    int lg = 1;
+    while ((1 << lg) < t) ++lg;
+    mmk::SellT<T>& o = d.lanes[lg - 1];
+    if (o.sptr) return;
+    std::vector<int> sptr(ns + 1, 0);
+    for (int s = 0; s < ns; ++s) {
+      int w = 0;
+      for (int r = per * s; r < std::min(A.n_rows, per * (s + 1)); ++r) w = std::max(w, (A.ptr[r + 1] - A.ptr[r] + t - 1) / t);
+      sptr[s + 1] = sptr[s] + 64 * ((w + 1) / 2);  // paired entries (mmk::SellT)
+    }
+    std::vector<int> col(sptr[ns], 0);
+    std::vector<double> val(sptr[ns], 0.0);
+    for (int r = 0; r < A.n_rows; ++r) {
+      const int s = r / per, w2 = (sptr[s + 1] - sptr[s]) / 32, len = A.ptr[r + 1] - A.ptr[r];
+      for (int k = 0; k < t * w2; ++k) {
+        const size_t at = (size_t)sptr[s] + 64 * (k / t / 2) + 2 * (r % per * t + k % t) + k / t % 2;
+        if (len > 0) col[at] = A.col[A.ptr[r] + std::min(k, len - 1)];  // padding: value 0, a column of the row
+        if (k < len) val[at] = A.val[A.ptr[r] + k];
+      }
+    }
+    o.n = A.n_rows;
+    o.sptr = upload(sptr);
+    o.col = upload(col);
+    o.val = upload_as<T>(val);
   }
   // sliced ELL (mmk::SellT): slices of 32 rows, entries paired, padding with value 0 and a valid column
   template <class T>
@@ -1063,10 +1102,11 @@ template <class T>
 mmk::POp<T> persistent_op(const DevMatT<T>& M) {
   mmk::POp<T> o{};
   while ((1 << o.lg) < M.tpr) ++o.lg;
-  o.n = M.tpr == 1 ? M.s.n : M.c.n;
-  o.ptr = M.tpr == 1 ? M.s.sptr : M.c.ptr;
-  o.col = M.tpr == 1 ? M.s.col : M.c.col;
-  o.val = M.tpr == 1 ? M.s.val : M.c.val;
+  const mmk::SellT<T>& s = o.lg == 0 ? M.s : M.lanes[o.lg - 1];
+  o.n = s.n;
+  o.ptr = s.sptr;
+  o.col = s.col;
+  o.val = s.val;
   return o;
 }
 
@@ -1165,7 +1205,7 @@ int persistent_args(mm_problem* h, SolverT<TP>& S, SolverT<TV>& F, mmk::PcgArgs<
   if (fused) {
     auto& c = F.lv[L - 2];
     mmk::PStep<TV>& sa = add(mmk::PS_COARSE_A, F.Tm.n);
-    sa.A = mmk::POp<TV>{F.Tm.n, 5, F.Tm.ptr, F.Tm.col, F.Tm.val};
+    sa.A = mmk::POp<TV>{F.Tm.n, 5, F.Tml.sptr, F.Tml.col, F.Tml.val};
     sa.x = c.b;
     sa.y = F.tvec;
     mmk::PStep<TV>& sb = add(mmk::PS_COARSE_B, (F.fn + 32 / mmk::CB_LANES - 1) / (32 / mmk::CB_LANES));
@@ -2994,6 +3034,12 @@ void build_fused_coarse(mm_problem* h, SolverT<T>& S, int precond_type) {
   S.Tm.col = h->upload(A.col);
   S.Tm.val = h->upload_as<T>(fc.tv);
   S.Tm_nnz = A.nnz();
+  DevMatT<T> lanes;
+  lanes.tpr = mmk::CA_LANES;
+  mm::HostCSR Tm = A;
+  Tm.val.assign(fc.tv.begin(), fc.tv.end());
+  h->upload_lanes<T>(Tm, lanes);
+  S.Tml = lanes.lanes[4];
   S.W = h->upload_as<T>(fc.W);
   S.Z = h->upload_as<T>(fc.Z);
   S.tvec = h->alloc<T>(n);
@@ -3916,6 +3962,7 @@ void tune_csr(mm_problem* h, SolverT<T>& S, DevMatT<T>& M, const mm::HostCSR& ho
   std::string times;
   for (int t : {1, 2, 4, 8, 16, 32}) {
     M.tpr = t;
+    h->upload_lanes<T>(host, M);
     const float ms = vcycle_ms<T>(h, S, reps);
     times += (times.empty() ? "" : ",") + std::to_string(1e3 * ms);
     if (t == before) before_ms = ms;
@@ -4187,16 +4234,29 @@ int mm_set_option(mm_problem* h, int option, int value) {
   if (option == MM_OPT_CSR_LANES) {
     if (value != 2 && value != 4 && value != 8 && value != 16 && value != 32) return MM_ERR_ARG;
     if (!h->poisson_built) return MM_ERR_STATE;
-    auto set_all = [&](auto& S) {
-      for (auto& c : S.lv)
-        for (auto* M : {&c.A, &c.R, &c.P, &c.Rf})
-          if (M->c.n > 0 && M->tpr != 1) M->tpr = value;
-      drop_graph(S);
-    };
-    set_all(h->s64);
-    set_all(h->s32);
-    h->drop_inner_graphs();
-    return MM_OK;
+    return guarded(h, [&] {
+      auto set_all = [&](auto& S) {
+        const int L = (int)S.lv.size();
+        for (int l = 0; l < L; ++l) {
+          auto& c = S.lv[l];
+          auto set = [&](auto& M, const mm::HostCSR& host) {
+            if (M.c.n == 0 || M.tpr == 1) return;
+            M.tpr = value;
+            h->upload_lanes(host, M);
+          };
+          set(c.A, h->amg_h[l].A);
+          if (l == L - 1) continue;
+          set(c.R, h->amg_h[l].R);
+          set(c.P, h->amg_h[l].P);
+          if (c.Rf.nnz > 0) set(c.Rf, h->rf_host[l]);
+        }
+        drop_graph(S);
+      };
+      set_all(h->s64);
+      set_all(h->s32);
+      h->drop_inner_graphs();
+      return MM_OK;
+    });
   }
   if (option == MM_OPT_COARSE_CYCLE) {
     if (value < 0 || value > 3) return MM_ERR_ARG;

@@ -25,7 +25,8 @@ constexpr int PSTEPS = 4 * PLEV + 6;
 constexpr int CHUNK = BS * ILP;  // rows of a separate kernel's block
 constexpr int WPB = BS / 32;     // its warps
 
-// an operator: lg == 0 sliced ELL (ptr: slice pointers), else compressed rows read by 1 << lg lanes
+// an operator in sliced ELL (ptr: slice pointers): a row to a lane (lg == 0), or dealt out over 1 << lg lanes
+// (upload_lanes)
 template <class T>
 struct POp {
   int n, lg;
@@ -233,51 +234,46 @@ __device__ __forceinline__ void psell2_df(const SellDF& A, const float* z, int r
   }
 }
 
-// FP64 products leave by branches on a count that the whole warp shares, since a predicated-off FP64 operation
-// still holds the FP64 pipe for its 16 clocks, eight of them for the two or three entries of a prolongation's
-// lane (lanes without an entry add zero to their sum): 59k rows' prolongation 10.6k -> 8.7k clocks, their whole
-// solve 787 -> 750 us.  FP32 products stay predicated (by branches their solves are 1-2 % slower).
+// A slice of a row dealt out over 1 << lg lanes, eight entries of a lane in flight; the row's sum in all its lanes.
+// FP64 products leave by branches on the slice's width: a predicated-off FP64 operation still holds the FP64 pipe
+// for its 16 clocks, eight of them for the two or three entries of a prolongation's lane.
 template <class T>
-__device__ __forceinline__ T pcsr_row(const int* __restrict__ ptr, const int* __restrict__ col,
-                                      const T* __restrict__ val, const T* x, int row, bool valid, int lane, int lg) {
-  constexpr int U = 8;
-  const int tpr = 1 << lg;
+__device__ __forceinline__ T planes(const POp<T>& A, const T* x, int s) {
+  using P2 = typename Pair<T>::type;
+  constexpr int U = 4;
+  const int lane = threadIdx.x & 31;
+  int at = __ldg(A.ptr + s);
+  int left = (__ldg(A.ptr + s + 1) - at) >> 6;
+  at += 2 * lane;
   T acc = T(0);
-  int k0 = 0, e = 0;
-  if (valid) {
-    k0 = __ldg(ptr + row) + lane;
-    e = __ldg(ptr + row + 1);
-  }
-  int left = __reduce_max_sync(0xffffffffu, e > k0 ? (e - k0 + tpr - 1) >> lg : 0);
 #pragma unroll 1
-  for (; left > 0; left -= U, k0 += U * tpr) {
-    int c[U] = {};  // defined on every path: a register that only predicated loads write stays live
-    T v[U] = {}, g[U] = {};  // through the whole kernel
+  for (; left > 0; left -= U, at += 64 * U) {
+    int2 c[U] = {};  // defined on every path: a register that only predicated loads write stays live
+    P2 v[U] = {};    // through the whole kernel
+    T g[U][2] = {};
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (k0 + u * tpr < e) {
-        c[u] = __ldg(col + k0 + u * tpr);
-        v[u] = __ldg(val + k0 + u * tpr);
+      if (u < left) {
+        c[u] = __ldg(reinterpret_cast<const int2*>(A.col + at + 64 * u));
+        v[u] = __ldg(reinterpret_cast<const P2*>(A.val + at + 64 * u));
       }
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (k0 + u * tpr < e) g[u] = x[c[u]];
-    if constexpr (sizeof(T) == 8) {
-      do {
-#define PMADD(K)         \
-  if (K >= left) break; \
-  acc = fmaT<T>(v[K], g[K], acc);
-        PMADD(0) PMADD(1) PMADD(2) PMADD(3) PMADD(4) PMADD(5) PMADD(6) PMADD(7)
+      if (u < left) {
+        g[u][0] = x[c[u].x];
+        g[u][1] = x[c[u].y];
+      }
+    do {
+#define PMADD(K)                             \
+  if (K >= left) break;                     \
+  acc = fmaT<T>(v[K].x, g[K][0], acc);       \
+  acc = fmaT<T>(v[K].y, g[K][1], acc);
+      PMADD(0) PMADD(1) PMADD(2) PMADD(3)
 #undef PMADD
-      } while (false);
-    } else {
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (k0 + u * tpr < e) acc = fmaT<T>(v[u], g[u], acc);
-    }
+    } while (false);
   }
 #pragma unroll 1
-  for (int o = tpr >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  for (int o = 1 << A.lg >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   return acc;
 }
 
@@ -308,13 +304,11 @@ __device__ __forceinline__ void prows(const PStep<T>& st, int lo, int hi) {
         if ((q ? r1 : r0) < A.n) prow_out<T>(st, q ? r1 : r0, ax[q]);
     }
   } else {  // units of a warp's rows
-    const int l = lane & ((1 << A.lg) - 1);
 #pragma unroll 1
     for (int u = lo + wid; u < hi; u += PW) {
+      const T ax = planes<T>(A, x, u);
       const int row = (u << (5 - A.lg)) + (lane >> A.lg);
-      const bool valid = row < A.n;
-      const T ax = pcsr_row<T>(A.ptr, A.col, A.val, x, row, valid, l, A.lg);
-      if (valid && l == 0) prow_out<T>(st, row, ax);
+      if (row < A.n && (lane & ((1 << A.lg) - 1)) == 0) prow_out<T>(st, row, ax);
     }
   }
 }
@@ -592,7 +586,7 @@ __device__ __forceinline__ void pcoarse_a(const PcgArgs<TP, TV>& a, const PStep<
     const int lane = tb & 31;
 #pragma unroll 1
     for (int row = lo + (tb - BS) / 32; row < hi; row += PW - WPB) {
-      const TV acc = pcsr_row<TV>(st.A.ptr, st.A.col, st.A.val, b, row, true, lane, 5);
+      const TV acc = planes<TV>(st.A, b, row);
       if (lane == 0) st.y[row] = acc;
     }
   }

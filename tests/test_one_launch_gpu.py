@@ -62,6 +62,25 @@ def test_one_launch_equals_separate_kernels(cuda_ok, mesh, precision):
     assert U is not None and np.abs(U).max() > 0
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32_precond"])
+def test_rows_dealt_out_over_every_number_of_lanes(cuda_ok, precision):
+    """Its operators are laid out for their lanes; the separate kernels read compressed rows."""
+    s = _setup(MESHES["ragged"])
+    prob = fem_utils.make_problem(s)
+    if precision != "fp64":
+        prob.set_precision(precision)
+    prob.build_poisson(1e-12, "amgcl")
+    m = syn.initial_state(s.N, seed=8, amplitude=0.3)
+    for lanes in (2, 4, 8, 16, 32):
+        prob.set_option("csr_lanes", lanes)
+        out = []
+        for graph in (1, 0):
+            prob.set_option("graph", graph)
+            out.append(prob.solve_u(m, np.zeros(s.N), 1e-10))
+        assert out[0][1:] == out[1][1:] and out[0][3] == 0
+        assert np.array_equal(out[0][0], out[1][0])
+
+
 def test_solves_in_flight_share_the_device_and_keep_their_bits(cuda_ok):
     """Several threads' solves: the number in flight changes how each runs, not what it returns."""
     s = _setup(MESHES["ragged"])
