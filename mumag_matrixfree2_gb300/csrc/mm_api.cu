@@ -95,6 +95,8 @@ struct DevMatT {
 template <class T>
 struct LevelT {
   DevMatT<T> A, P, R;
+  DevMatT<T> G;      // folded prolongation (mm::folded_prolongation), empty when not formed; x2 of the next level
+                     // lies behind b (level 0: r) for it
   DevMatT<T> Rf;     // fused restriction R (I - A S) (levels below the coarsest), empty when not formed
   T* s = nullptr;    // smoother diagonal (SPAI0, or omega/(diag+eps) for Jacobi)
   T* b = nullptr;    // right-hand side (levels >= 1)
@@ -292,6 +294,7 @@ struct mm_problem {
   int sa_theta_e3 = 0;           // MM_OPT_SA_THETA_E3 (0: the setup's default)
   int sa_factor_e3 = 0;          // MM_OPT_SA_FACTOR_E3 (0: the setup's default)
   int sa_filter_e6 = 0;          // MM_OPT_SA_FILTER_E6 (0: the setup's default, < 0: no filtering)
+  std::vector<mm::HostCSR> g_host;   // folded prolongations, formed with rf_host
   std::vector<mm::HostCSR> rf_host;  // fused restrictions R_l (I - A_l S_l), formed for smoother rf_prec
   int rf_prec = -1;
   // host factors shared by the FP64 and FP32 copies of the hierarchy (formed once, O(nc^3) and
@@ -792,6 +795,17 @@ double mat_bytes(const DevMatT<T>& M) {
   return (double)M.nnz * (4.0 + sizeof(T)) + 4.0 * ptrs;
 }
 
+// level l's prolongation and post-smoothing run as one product with G (its pre-smoothing is in it and in the
+// fused restriction)
+template <class T>
+bool folded(const mm_problem* h, const SolverT<T>& S, int l) {
+  const int L = (int)S.lv.size();
+  const int bit = sizeof(T) == 8 ? 0 : 1;
+  return ((h->fuse_restrict >> bit) & 1) && S.lv[l].G.nnz > 0 && S.lv[l].Rf.nnz > 0 &&
+         l < (S.fused && ((h->coarse_fuse >> bit) & 1) ? L - 2 : L - 1) &&
+         (l > 0 || (int64_t)grid_ilp(h->N) * mmk::CHUNK >= h->N);  // pfold0 makes one round of the grid's blocks
+}
+
 // ---------------------------------------------------------------------------------------------
 // V-cycle (enqueue only).  Level 0's pre-smoothed iterate lv[0].x must already hold s0 .* r.
 // in_loop: the level-0 residual is skipped once the solve has converged.
@@ -806,12 +820,13 @@ void enqueue_vcycle(mm_problem* h, SolverT<T>& S, const T* r, T* z, bool in_loop
   const bool fuse = S.fused && ((h->coarse_fuse >> (sizeof(T) == 8 ? 0 : 1)) & 1);
   const int Ld = fuse ? L - 2 : L - 1;  // levels l < Ld compute a residual and restrict it
   const bool fr_on = (h->fuse_restrict >> (sizeof(T) == 8 ? 0 : 1)) & 1;
+  auto fold = [&](int l) { return folded(h, S, l) && (l > 0 || r == S.r); };
   // b_{l+1} = R_l res (res = b_l - A_l x_l), and the pre-smoothing x_{l+1} = s_{l+1} b_{l+1} unless
   // level l+1 has none
   auto restrict_into = [&](int l, const DevMatT<T>& M, const T* in, double mbytes) {
     auto& c = lv[l];
     auto& nx = lv[l + 1];
-    const bool no_pre = (l + 1 == L - 1) || (fuse && l + 1 == L - 2);
+    const bool no_pre = (l + 1 == L - 1) || (fuse && l + 1 == L - 2) || fold(l + 1);
     const double rbytes = mbytes + w * c.n + (no_pre ? 1.0 : 3.0) * w * nx.n;
     tagged<T>(h, MM_PROF_RESTRICT, l, rbytes, [&] {
       if (M.tpr == 1) {
@@ -828,7 +843,7 @@ void enqueue_vcycle(mm_problem* h, SolverT<T>& S, const T* r, T* z, bool in_loop
   // restriction at level 1, fused coarse correction, compressed rows on level 1)
   const bool cc_on = ((h->coarse_cycle >> (sizeof(T) == 8 ? 0 : 1)) & 1) && fuse && fr_on && L == 4 &&
                      lv[0].Rf.nnz > 0 && lv[1].Rf.nnz > 0 && lv[1].Rf.tpr > 1 && lv[1].P.tpr > 1 &&
-                     lv[1].A.tpr > 1 && S.bar && S.coop_grid > 0;
+                     lv[1].A.tpr > 1 && (!fold(1) || lv[1].G.tpr > 1) && S.bar && S.coop_grid > 0;
   for (int l = 0; l < (cc_on ? 1 : Ld); ++l) {
     auto& c = lv[l];
     if (fr_on && c.Rf.nnz > 0) {
@@ -858,6 +873,10 @@ void enqueue_vcycle(mm_problem* h, SolverT<T>& S, const T* r, T* z, bool in_loop
     cc.tpr_rf1 = l1.Rf.tpr;
     cc.tpr_p1 = l1.P.tpr;
     cc.tpr_a1 = l1.A.tpr;
+    if (fold(1)) {
+      cc.G1 = l1.G.c;
+      cc.tpr_g1 = l1.G.tpr;
+    }
     cc.b1 = l1.b;
     cc.x1 = l1.x;
     cc.s1 = l1.s;
@@ -870,7 +889,7 @@ void enqueue_vcycle(mm_problem* h, SolverT<T>& S, const T* r, T* z, bool in_loop
     cc.tvec = S.tvec;
     cc.zvec = S.zvec;
     cc.x2_2 = l2.x2;
-    const double bytes = mat_bytes(l1.Rf) + mat_bytes(l1.P) + mat_bytes(l1.A) + 4.0 * ((double)S.Tm.n + 1.0) +
+    const double bytes = mat_bytes(l1.Rf) + (fold(1) ? mat_bytes(l1.G) : mat_bytes(l1.P) + mat_bytes(l1.A)) + 4.0 * ((double)S.Tm.n + 1.0) +
                          (4.0 + w) * (double)S.Tm_nnz + 2.0 * w * (double)S.fc * S.fn + w * 7.0 * l1.n +
                          w * 6.0 * l2.n;
     tagged<T>(h, MM_PROF_COARSE_CYCLE, 1, bytes, [&] {
@@ -910,6 +929,16 @@ void enqueue_vcycle(mm_problem* h, SolverT<T>& S, const T* r, T* z, bool in_loop
   }
   for (int l = (cc_on ? 0 : fuse ? L - 3 : L - 2); l >= 0; --l) {
     auto& c = lv[l];
+    if (fold(l)) {
+      tagged<T>(h, MM_PROF_PROLONG, l, mat_bytes(c.G) + w * lv[l + 1].n + 2.0 * w * c.n,
+                [&] { spmv<0, T>(h, c.G, l == 0 ? r : c.b, nullptr, nullptr, l == 0 ? z : c.x2, done); });
+      if (l > 0) continue;
+      tagged<T>(h, MM_PROF_SMOOTH0, 0, 2.0 * w * c.n, [&] {
+        launch(h, mmk::k_rz<T>, grid_ilp(c.n), BS, c.n, r, z, sc, h->d_part, done, z64, red_kshift(c.n));
+        LAUNCH_CHECK();
+      });
+      continue;
+    }
     tagged<T>(h, MM_PROF_PROLONG, l, mat_bytes(c.P) + w * lv[l + 1].n + 2.0 * w * c.n,
               [&] { spmv<3, T>(h, c.P, lv[l + 1].x2, c.x, nullptr, c.x, done); });  // x += P e
     if (l == 0) {
@@ -1165,7 +1194,7 @@ int persistent_args(mm_problem* h, SolverT<TP>& S, SolverT<TV>& F, mmk::PcgArgs<
   a.p = S.p;
   a.Ap = S.Ap;
   a.s0 = F.lv[0].s;
-  a.xv = F.lv[0].x;
+  a.xv = folded(h, F, 0) ? nullptr : F.lv[0].x;
   a.rv = F.r;
   a.z = F.z;
   a.Z = F.Z;
@@ -1199,7 +1228,7 @@ int persistent_args(mm_problem* h, SolverT<TP>& S, SolverT<TV>& F, mmk::PcgArgs<
     const TV* bl = l == 0 ? F.r : c.b;
     const bool rf = use_rf && c.Rf.nnz > 0;
     if (!rf) rows(mmk::PS_RESID, c.A, c.x, bl, nullptr, c.res, nullptr);
-    const bool no_pre = (l + 1 == L - 1) || (fused && l + 1 == L - 2);
+    const bool no_pre = (l + 1 == L - 1) || (fused && l + 1 == L - 2) || folded(h, F, l + 1);
     rows(mmk::PS_RESTRICT, rf ? c.Rf : c.R, rf ? bl : c.res, nullptr, nx.s, nx.b, no_pre ? nullptr : nx.x);
   }
   if (fused) {
@@ -1227,10 +1256,21 @@ int persistent_args(mm_problem* h, SolverT<TP>& S, SolverT<TV>& F, mmk::PcgArgs<
   }
   for (int l = fused ? L - 3 : L - 2; l >= 0; --l) {
     auto& c = F.lv[l];
+    if (folded(h, F, l)) {
+      if (l > 0) {
+        rows(mmk::PS_PROLONG, c.G, c.b, nullptr, nullptr, c.x2, nullptr);
+      } else {
+        mmk::PStep<TV>& st = add(mmk::PS_FOLD0, parts);
+        st.A = persistent_op(c.G);
+        st.x = F.r;
+        st.y = F.z;
+      }
+      continue;
+    }
     rows(mmk::PS_PROLONG, c.P, F.lv[l + 1].x2, c.x, nullptr, c.x, nullptr);
     if (l > 0) rows(mmk::PS_SMOOTH, c.A, c.x, c.b, c.s, c.x2, nullptr);
   }
-  add(mmk::PS_SMOOTH0, parts).A = persistent_op(F.lv[0].A);
+  if (!folded(h, F, 0)) add(mmk::PS_SMOOTH0, parts).A = persistent_op(F.lv[0].A);
   add(mmk::PS_DIR, parts);
   add(mmk::PS_STEP, parts);
   return blocks;
@@ -1257,6 +1297,8 @@ void launch_persistent(mm_problem* h, SolverT<TP>& S, SolverT<TV>& F, double tol
   cfg.blockDim = dim3(mmk::PT);
   const int parts = a.kshift ? (a.G * mmk::WPB) >> a.kshift : 0;  // a block folds its share of these and of b.b's
   cfg.dynamicSmemBytes = (size_t)((std::max(parts, a.Gdot) + blocks - 1) / blocks) * BS * sizeof(double);
+  if (folded(h, F, 0))  // and keeps its rows of z
+    cfg.dynamicSmemBytes += (size_t)((((a.G * mmk::WPB) >> a.kshift) + blocks - 1) / blocks << a.kshift) * 64 * sizeof(TV);
   cfg.stream = h->st;
   cfg.attrs = at;
   cfg.numAttrs = 1;
@@ -3049,6 +3091,20 @@ void build_fused_coarse(mm_problem* h, SolverT<T>& S, int precond_type) {
   S.fused = true;
 }
 
+// a level's rows of the vector that G takes, before the coarse correction's
+inline int fold_offset(int n) { return (n + 31) / 32 * 32; }
+
+// Levels whose prolongation and post-smoothing are folded into one product.  It has about half as many entries again
+// (17 against 10 a row on level 0, 56 against 37 on level 1) but saves a phase of the one-launch PCG (7k clocks and
+// more: a barrier and a chain of dependent loads), or a launch, and the pre-smoothed iterate.  A solve without, with
+// it on the levels from 1, and on all: 1,331 rows 306 and 267 us; 59,319 rows 726, 688 and 665 (FP32 V-cycle 677, 652
+// and 605); 357,911 rows 1833, 1805 and 1847 (1623, 1620 and 1659); 1,601,613 rows 5.97 and 5.88 ms (4.96 and 5.08,
+// where level 1 has 222,818 rows).
+template <class T>
+bool fold_rows(int l, int64_t n) {
+  return n <= (l == 0 ? 131072 : sizeof(T) == 8 ? 262144 : 65536);
+}
+
 // Upload the hierarchy in precision T and allocate the solver's vectors.
 template <class T>
 void build_solver(mm_problem* h, SolverT<T>& S, const mm::HostCSR& A, bool amg, int precond_type) {
@@ -3069,15 +3125,20 @@ void build_solver(mm_problem* h, SolverT<T>& S, const mm::HostCSR& A, bool amg, 
         sd[i] = precond_type == MM_PRECOND_AMGCL ? hl.spai0[i] : 0.6667 / (hl.diag[i] + 1e-30);
       dl.s = h->upload_as<T>(sd);
     }
-    dl.b = h->alloc<T>(dl.n);
+    // b, and the next level's x2 behind it (level 0: behind r)
+    T* const b = h->alloc<T>(fold_offset(dl.n) + (l < L - 1 ? (size_t)h->amg_h[l + 1].A.n_rows : 0));
+    (l == 0 ? S.r : dl.b) = b;
+    if (l == 0) dl.b = h->alloc<T>(dl.n);
+    if (l == 0) dl.x2 = h->alloc<T>(dl.n);
+    if (l < L - 1) S.lv[l + 1].x2 = b + fold_offset(dl.n);
     dl.x = h->alloc<T>(dl.n);
-    dl.x2 = h->alloc<T>(dl.n);
     dl.res = h->alloc<T>(dl.n);
   }
   if (amg && L >= 2) {
     // fused restrictions R_l (I - A_l S_l) with the smoother of this hierarchy, formed once in FP64
     if ((int)h->rf_host.size() != L - 1 || h->rf_prec != precond_type) {
       h->rf_host.assign(L - 1, mm::HostCSR{});
+      h->g_host.assign(L - 1, mm::HostCSR{});
       for (int l = 0; l < L - 1; ++l) {
         const mm::AmgLevel& hl = h->amg_h[l];
         std::vector<double> sd(hl.A.n_rows);
@@ -3090,7 +3151,21 @@ void build_solver(mm_problem* h, SolverT<T>& S, const mm::HostCSR& A, bool amg, 
       h->rf_prec = precond_type;
       for (mm::AmgLevel& hl : h->amg_h) hl.RA = mm::HostCSR{};  // its one use is above
     }
-    for (int l = 0; l < L - 1; ++l) S.lv[l].Rf = h->upload_mat<T>(h->rf_host[l]);
+    for (int l = 0; l < L - 1; ++l) {
+      S.lv[l].Rf = h->upload_mat<T>(h->rf_host[l]);
+      if (!fold_rows<T>(l, h->amg_h[l].A.n_rows)) continue;
+      const mm::AmgLevel& hl = h->amg_h[l];
+      mm::HostCSR& g = h->g_host[l];
+      if (g.n_rows == 0) {
+        std::vector<double> sd(hl.A.n_rows);
+        for (int i = 0; i < hl.A.n_rows; ++i)
+          sd[i] = precond_type == MM_PRECOND_AMGCL ? hl.spai0[i] : 0.6667 / (hl.diag[i] + 1e-30);
+        g = mm::folded_prolongation(hl.A, hl.P, sd, fold_offset(hl.A.n_rows));
+      }
+      // level 0 from 16Ki rows on by one thread a row: 59,319 rows, a V-cycle with 1, 2, 4 and 8 lanes 38.4, 39.0,
+      // 39.2 and 40.1 us
+      S.lv[l].G = h->upload_mat<T>(g, l == 0 && g.n_rows >= 16384);
+    }
   }
   if (amg) {
     const mm::HostCSR& Ac = h->amg_h.back().A;
@@ -3104,7 +3179,7 @@ void build_solver(mm_problem* h, SolverT<T>& S, const mm::HostCSR& A, bool amg, 
     for (int i = 0; i < h->N; ++i) jac[i] = 1.0 / (dg[i] + 1e-30);
     S.jac = h->upload_as<T>(jac);
   }
-  S.r = h->alloc<T>(h->N);
+  if (L == 0) S.r = h->alloc<T>(h->N);
   S.z = h->alloc<T>(h->N);
   S.p = h->alloc<T>(h->N);
   S.Ap = h->alloc<T>(h->N);
@@ -3950,10 +4025,11 @@ float vcycle_ms(mm_problem* h, SolverT<T>& S, int reps) {
 
 // Lanes per row of one compressed-row operator: every candidate is timed in context, as the time of
 // whole V-cycles or PCG iterations (cache state and neighbours are those of a solve; an operator timed
-// alone, L2-hot, prefers fewer lanes than it should), and the fastest is kept.
+// alone, L2-hot, prefers fewer lanes than it should), and the fastest is kept.  An operator that the solve
+// does not read keeps its lanes, with one time for all.
 template <class T>
 void tune_csr(mm_problem* h, SolverT<T>& S, DevMatT<T>& M, const mm::HostCSR& host, int reps, const char* tag,
-              int level, std::string& rep) {
+              int level, bool used, std::string& rep) {
   if (M.c.n == 0) return;  // sliced ELL only (level 0)
   if (!M.s.sptr) h->upload_sell<T>(host, M);  // the one-thread-per-row candidate
   const int before = M.tpr;
@@ -3961,11 +4037,13 @@ void tune_csr(mm_problem* h, SolverT<T>& S, DevMatT<T>& M, const mm::HostCSR& ho
   float best_ms = 1e30f, before_ms = 1e30f;
   std::string times;
   for (int t : {1, 2, 4, 8, 16, 32}) {
-    M.tpr = t;
-    h->upload_lanes<T>(host, M);
-    const float ms = vcycle_ms<T>(h, S, reps);
+    if (used) {
+      M.tpr = t;
+      h->upload_lanes<T>(host, M);
+    }
+    const float ms = used || t == 1 ? vcycle_ms<T>(h, S, reps) : before_ms;
     times += (times.empty() ? "" : ",") + std::to_string(1e3 * ms);
-    if (t == before) before_ms = ms;
+    if (t == before || !used) before_ms = ms;
     if (ms < best_ms) {
       best_ms = ms;
       best = t;
@@ -3986,11 +4064,15 @@ void tune_solver(mm_problem* h, SolverT<T>& S, int reps, std::string& rep) {
   const int L = (int)S.lv.size();
   for (int l = 0; l < L; ++l) {
     auto& c = S.lv[l];
-    if (l > 0) tune_csr<T>(h, S, c.A, h->amg_h[l].A, reps, "A", l, rep);
+    const int bit = sizeof(T) == 8 ? 0 : 1;
+    const bool rf = ((h->fuse_restrict >> bit) & 1) && c.Rf.nnz > 0;
+    const bool on = l < (S.fused && ((h->coarse_fuse >> bit) & 1) ? L - 2 : L - 1), g = folded(h, S, l);
+    if (l > 0) tune_csr<T>(h, S, c.A, h->amg_h[l].A, reps, "A", l, on && !(rf && g), rep);
     if (l < L - 1) {
-      tune_csr<T>(h, S, c.R, h->amg_h[l].R, reps, "R", l, rep);
-      tune_csr<T>(h, S, c.P, h->amg_h[l].P, reps, "P", l, rep);
-      if (c.Rf.nnz > 0 && (int)h->rf_host.size() > l) tune_csr<T>(h, S, c.Rf, h->rf_host[l], reps, "Rf", l, rep);
+      tune_csr<T>(h, S, c.R, h->amg_h[l].R, reps, "R", l, on && !rf, rep);
+      tune_csr<T>(h, S, c.P, h->amg_h[l].P, reps, "P", l, on && !g, rep);
+      if (c.Rf.nnz > 0 && (int)h->rf_host.size() > l) tune_csr<T>(h, S, c.Rf, h->rf_host[l], reps, "Rf", l, on && rf, rep);
+      if (c.G.nnz > 0) tune_csr<T>(h, S, c.G, h->g_host[l], reps, "G", l, on && g, rep);
     }
   }
   drop_graph(S);
@@ -4249,6 +4331,7 @@ int mm_set_option(mm_problem* h, int option, int value) {
           set(c.R, h->amg_h[l].R);
           set(c.P, h->amg_h[l].P);
           if (c.Rf.nnz > 0) set(c.Rf, h->rf_host[l]);
+          if (c.G.nnz > 0) set(c.G, h->g_host[l]);
         }
         drop_graph(S);
       };

@@ -942,8 +942,8 @@ __global__ void __launch_bounds__(BS) k_coarse_b(int n, int nc, const T* __restr
 // ------------------------------------------------------------------------------------------
 // The V-cycle's levels 1 .. 3 of a four-level hierarchy in one cooperative launch (fused restriction
 // at level 1, fused coarse correction on levels 2 .. 3): b2 = Rf1 b1 | t = T b2, z = Z b2 |
-// x2_2 = t + W z | x1 += P1 x2_2 | x2_1 = x1 + s1 (b1 - A1 x1), five stages separated by grid
-// barriers instead of five launches.  Every row is computed exactly as by the separate kernels (same
+// x2_2 = t + W z | x1 += P1 x2_2 | x2_1 = x1 + s1 (b1 - A1 x1) (the last two folded: x2_1 = G1 [b1; x2_2]),
+// stages separated by grid barriers instead of launches.  Every row is computed exactly as by the separate kernels (same
 // lanes per row, same order), so the V-cycle's result is bit-identical.
 // ------------------------------------------------------------------------------------------
 struct GridBar {
@@ -1011,8 +1011,8 @@ __device__ __forceinline__ void csr_rows_tpr(int tpr, const CsrT<T>& A, const T*
 
 template <class T>
 struct CoarseCycle {
-  CsrT<T> Rf1, P1, A1, Tm;
-  int tpr_rf1, tpr_p1, tpr_a1;
+  CsrT<T> Rf1, P1, A1, Tm, G1;
+  int tpr_rf1, tpr_p1, tpr_a1, tpr_g1;
   const T* b1;  // level-1 right-hand side (the restricted level-0 residual)
   T* x1;        // level-1 iterate (pre-smoothed s1 b1 on entry)
   const T* s1;
@@ -1034,6 +1034,10 @@ __global__ void __launch_bounds__(BS) k_coarse_cycle(CoarseCycle<T> c, GridBar* 
   grid_sync(bar, sc);
   coarse_b_rows<T>(c.Tm.n, c.nc, c.W, c.tvec, c.zvec, c.x2_2, (int)blockIdx.x, (int)gridDim.x);
   grid_sync(bar, sc);
+  if (c.G1.n) {  // folded: from b1 and, behind it, x2_2
+    csr_rows_tpr<0, T>(c.tpr_g1, c.G1, c.b1, nullptr, nullptr, c.x2_1);
+    return;
+  }
   csr_rows_tpr<3, T>(c.tpr_p1, c.P1, c.x2_2, c.x1, nullptr, c.x1);
   grid_sync(bar, sc);
   csr_rows_tpr<2, T>(c.tpr_a1, c.A1, c.x1, c.b1, c.s1, c.x2_1);
@@ -1067,6 +1071,29 @@ __global__ void __launch_bounds__(BS) k_smooth_dot(SellT<T> A, const T* __restri
     }
   }
   if (part) chunk_finish(acc, sc, part, R_RZ, POST_RZ, kshift);
+}
+
+// r.z -> red[R_RZ] after the folded prolongation on level 0; y64 as in k_smooth_dot
+template <class T>
+__global__ void __launch_bounds__(BS) k_rz(int n, const T* __restrict__ r, const T* __restrict__ z, Scalars* sc,
+                                           double* part, const int* __restrict__ done, double* __restrict__ y64,
+                                           int kshift) {
+  pdl_entry();
+  if (done && *done) return;
+  Acc<T> acc;
+  ROW_LOOP(n) {
+    int row[ILP];
+    rows_of(rb, row);
+#pragma unroll
+    for (int q = 0; q < ILP; ++q) {
+      const int i = row[q];
+      if (i >= n) continue;
+      const T zi = z[i];
+      if (y64) y64[i] = (double)zi;
+      acc.add(r[i], zi);
+    }
+  }
+  chunk_finish(acc, sc, part, R_RZ, POST_RZ, kshift);
 }
 
 // condition of the graph's WHILE node: keep looping until done (bounded by maxiter + 2 trips)

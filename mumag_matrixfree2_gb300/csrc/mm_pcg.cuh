@@ -37,7 +37,7 @@ struct POp {
 
 // kinds of step.  Rows: PS_RESID y = b - A x; PS_RESTRICT y = A x and the coarse pre-smoothing y2 = s .* y
 // (y2 may be null); PS_PROLONG y = b + A x; PS_SMOOTH y = x + s .* (b - A x).
-enum PStepKind { PS_START, PS_DIR, PS_STEP, PS_SMOOTH0, PS_RESID, PS_RESTRICT, PS_PROLONG, PS_SMOOTH, PS_COARSE_A,
+enum PStepKind { PS_START, PS_DIR, PS_STEP, PS_SMOOTH0, PS_FOLD0, PS_RESID, PS_RESTRICT, PS_PROLONG, PS_SMOOTH, PS_COARSE_A,
                  PS_COARSE_B, PS_DENSE };
 
 template <class T>
@@ -283,7 +283,7 @@ __device__ __forceinline__ void prow_out(const PStep<T>& st, int i, T ax) {
   if (st.kind == PS_RESTRICT) {
     st.y[i] = ax;
     if (st.y2) st.y2[i] = st.s[i] * ax;
-  } else if (st.kind == PS_PROLONG) st.y[i] = st.b[i] + ax;
+  } else if (st.kind == PS_PROLONG) st.y[i] = st.b ? st.b[i] + ax : ax;
   else if (st.kind == PS_SMOOTH) st.y[i] = st.x[i] + st.s[i] * (st.b[i] - ax);
   else st.y[i] = st.b[i] - ax;
 }
@@ -385,6 +385,43 @@ __device__ __noinline__ void ptotal(PScal& ps, const double* part, int slot, int
   __syncwarp();
 }
 
+// A unit's sum: a partial of its own, or kept in shared memory for pparts_out, which folds a partial of eight units.
+template <class T>
+__device__ __forceinline__ void punit_out(Acc<T>& acc, double* pa, int kshift, int u) {
+  const int lane = threadIdx.x & 31;
+  if (kshift == 0) {
+    const double t = acc.warp_total();
+    if (lane == 0) pa[u] = t;
+  } else if constexpr (std::is_same<T, double>::value) {
+    s_unit[32 * u + lane] = acc.s;
+  } else {
+    const double t = acc.warp_total();
+    if (lane == 0) s_unit[u] = t;
+  }
+}
+
+template <class T>
+__device__ __forceinline__ void pparts_out(double* pa, int kshift, int nc) {
+  if (kshift == 0) return;
+  const int lane = threadIdx.x & 31;
+  __syncthreads();
+#pragma unroll 1
+  for (int c = threadIdx.x >> 5; c < nc; c += PW) {
+    double t;
+    if constexpr (std::is_same<T, double>::value) {
+      double u[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) u[j] = s_unit[32 * (8 * c + j) + lane];
+      t = warp_sum(fold8<false>(u));
+    } else {
+      t = 0.0;
+#pragma unroll 1
+      for (int j = 0; j < WPB; ++j) t += s_unit[WPB * c + j];
+    }
+    if (lane == 0) pa[c] = t;
+  }
+}
+
 // The steps with a reduction over level 0's rows, on vectors of T.  kind PS_START: r = b - A x, r.r;
 // PS_DIR: p = z + beta p, Ap = A z + beta Ap, p.Ap; PS_STEP: x += alpha p, r -= alpha Ap, r.r (both with
 // the V-cycle's input and its pre-smoothing xv = s0 .* r); PS_SMOOTH0: z = x + s0 .* (r - A x), r.z.
@@ -473,7 +510,7 @@ __device__ __forceinline__ void preduce(const PcgArgs<TP, TV>& a, int kind, PSca
           acc.add(ri, ri);
           const TV rf = (TV)ri;
           if (MP) a.rv[i] = rf;
-          a.xv[i] = a.s0[i] * rf;
+          if (a.xv) a.xv[i] = a.s0[i] * rf;
         } else if (INNER) {
           const T yi = e0[q] + e1[q] * (e2[q] - ax[q]);
           a.z[i] = (TV)yi;
@@ -481,34 +518,54 @@ __device__ __forceinline__ void preduce(const PcgArgs<TP, TV>& a, int kind, PSca
         }
       }
     }
-    if (kshift == 0) {
-      const double t = acc.warp_total();
-      if (lane == 0) pa[u] = t;
-    } else if constexpr (std::is_same<T, double>::value) {
-      s_unit[32 * u + lane] = acc.s;
-    } else {
-      const double t = acc.warp_total();
-      if (lane == 0) s_unit[u] = t;
-    }
+    punit_out(acc, pa, kshift, u);
   }
   meet();
-  if (kshift == 0) return;
+  pparts_out<T>(pa, kshift, nc);
+}
+
+// The folded prolongation on level 0, z = A [r; e] (e behind r in memory), and r.z.  The rows may be dealt out over lanes
+// (below 16Ki rows), and a block takes those of its partials, whose
+// sums it then forms in k_rz's order from shared memory.  Small problems only, so a unit is 64 rows (no second round
+// of a grid's blocks).
+template <class TP, class TV>
+__device__ __forceinline__ void pfold0(const PcgArgs<TP, TV>& a, const PStep<TV>& st, int c0, int nc) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const POp<TV> A = st.A;
+  const int n = A.n, lg = A.lg, kshift = a.kshift, U = nc << kshift;
+  double* const pa = a.part + (size_t)R_RZ * MAXG + c0;
+  TV* const s_z = reinterpret_cast<TV*>(s_unit + (kshift ? 32 * U : 0));
+  auto row0 = [&](int u, int q) {
+    const int ug = (c0 << kshift) + u;
+    return ug / WPB * CHUNK + 32 * (ug % WPB) + q * BS;
+  };
+#pragma unroll 1
+  for (int k = wid; k < U << (lg + 1); k += PW) {
+    const int g = k >> lg, sub = k & ((1 << lg) - 1), r0 = row0(g >> 1, g & 1) + (sub << (5 - lg));
+    if (r0 >= n) continue;
+    const TV ax = planes<TV>(A, st.x, r0 >> (5 - lg));
+    const int j = lane >> lg;
+    if (r0 + j < n && (lane & ((1 << lg) - 1)) == 0) {
+      st.y[r0 + j] = ax;
+      s_z[32 * g + (sub << (5 - lg)) + j] = ax;
+    }
+  }
+  TV r[2] = {};  // the first unit's, in flight over the barrier
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    if (wid < U && row0(wid, q) + lane < n) r[q] = st.x[row0(wid, q) + lane];
   __syncthreads();
 #pragma unroll 1
-  for (int c = wid; c < nc; c += PW) {
-    double t;
-    if constexpr (std::is_same<T, double>::value) {
-      double u[8];
+  for (int u = wid; u < U; u += PW) {
+    Acc<TV> acc;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) u[j] = s_unit[32 * (8 * c + j) + lane];
-      t = warp_sum(fold8<false>(u));
-    } else {
-      t = 0.0;
-#pragma unroll 1
-      for (int j = 0; j < WPB; ++j) t += s_unit[WPB * c + j];
+    for (int q = 0; q < 2; ++q) {
+      const int i = row0(u, q) + lane;
+      if (i < n) acc.add(u == wid ? r[q] : st.x[i], s_z[64 * u + 32 * q + lane]);
     }
-    if (lane == 0) pa[c] = t;
+    punit_out(acc, pa, kshift, u);
   }
+  pparts_out<TV>(pa, kshift, nc);
 }
 
 // b.b -> R_BB with k_dot's blocks (a partial of eight warps each)
@@ -529,29 +586,9 @@ __device__ __forceinline__ void pdot_bb(const PcgArgs<TP, TV>& a) {
           acc.add(bi, bi);
         }
       }
-    if constexpr (std::is_same<TP, double>::value) {
-      s_unit[32 * u + lane] = acc.s;
-    } else {
-      const double t = acc.warp_total();
-      if (lane == 0) s_unit[u] = t;
-    }
+    punit_out(acc, nullptr, 3, u);
   }
-  __syncthreads();
-#pragma unroll 1
-  for (int c = wid; c < nc; c += PW) {
-    double t;
-    if constexpr (std::is_same<TP, double>::value) {
-      double u[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) u[j] = s_unit[32 * (8 * c + j) + lane];
-      t = warp_sum(fold8<false>(u));
-    } else {
-      t = 0.0;
-#pragma unroll 1
-      for (int j = 0; j < WPB; ++j) t += s_unit[c * WPB + j];
-    }
-    if (lane == 0) a.part[(size_t)R_BB * MAXG + c0 + c] = t;
-  }
+  pparts_out<TP>(a.part + (size_t)R_BB * MAXG + c0, 3, nc);
   __syncthreads();
 }
 
@@ -631,6 +668,8 @@ __device__ __forceinline__ void pcg_run(const PcgArgs<TP, TV>& a, PScal& ps, con
       ptotal(ps, a.part, i == 1 ? R_R2 : kind == PS_DIR ? R_RZ : R_PAP, parts, it, a.maxiter, a.tol);
     if (kind >= PS_RESID && kind <= PS_SMOOTH) {
       prows<TV>(st, lo, hi);
+    } else if (kind == PS_FOLD0) {
+      pfold0(a, st, lo, hi - lo);
     } else if (kind == PS_COARSE_A) {
       pcoarse_a(a, st, ps.red[0], lo, hi);
     } else if (kind >= PS_COARSE_B) {

@@ -658,6 +658,50 @@ HostCSR fused_restriction_ra(const HostCSR& R, const HostCSR& RA, const std::vec
   return F;
 }
 
+HostCSR folded_prolongation(const HostCSR& A, const HostCSR& P, const std::vector<double>& s, int offset) {
+  const HostCSR AP = spgemm(A, P);
+  const int n = A.n_rows, nt = setup_threads(A.ptr[n] + AP.ptr[n]);
+  std::vector<std::vector<int>> tcol(nt);
+  std::vector<std::vector<double>> tval(nt);
+  std::vector<int> cnt(n + 1, 0);
+  parallel_chunks(n, nt, [&](int t, int64_t r0, int64_t r1) {
+    for (int64_t i = r0; i < r1; ++i) {
+      const size_t before = tcol[t].size();
+      auto put = [&](int c, double v) {
+        if (v == 0.0) return;
+        tcol[t].push_back(c);
+        tval[t].push_back(v);
+      };
+      bool diag = false;
+      for (int k = A.ptr[i]; k < A.ptr[i + 1]; ++k) {
+        const int j = A.col[k];
+        if (j > i && !diag) put((int)i, 2.0 * s[i]);  // no stored diagonal
+        diag = diag || j >= i;
+        put(j, (j == i ? 2.0 * s[i] : 0.0) - s[i] * A.val[k] * s[j]);
+      }
+      if (!diag) put((int)i, 2.0 * s[i]);
+      int a = P.ptr[i], b = AP.ptr[i];
+      const int ae = P.ptr[i + 1], be = AP.ptr[i + 1];
+      while (a < ae || b < be) {  // P - S A P, merging two sorted rows
+        const int ca = a < ae ? P.col[a] : P.n_cols, cb = b < be ? AP.col[b] : P.n_cols, c = std::min(ca, cb);
+        double v = 0.0;
+        if (ca == c) v += P.val[a++];
+        if (cb == c) v -= s[i] * AP.val[b++];
+        put(offset + c, v);
+      }
+      cnt[i + 1] = (int)(tcol[t].size() - before);
+    }
+  });
+  HostCSR G;
+  G.n_rows = n;
+  G.n_cols = offset + P.n_cols;
+  G.ptr.assign(n + 1, 0);
+  for (int i = 0; i < n; ++i) G.ptr[i + 1] = G.ptr[i] + cnt[i + 1];
+  concat_parallel(tcol, G.col);
+  concat_parallel(tval, G.val);
+  return G;
+}
+
 static std::vector<double> diag_of(const HostCSR& A) {
   std::vector<double> d(A.n_rows, 0.0);
   parallel_chunks(A.n_rows, setup_threads(A.n_rows), [&](int, int64_t r0, int64_t r1) {

@@ -130,6 +130,9 @@ std::vector<AmgLevel> build_amg(const HostCSR& A, const AmgParams& prm);
 HostCSR fused_restriction(const HostCSR& R, const HostCSR& A, const std::vector<double>& s);
 // the same from the product RA = R A: R - (R A) S, with no second sparse product
 HostCSR fused_restriction_ra(const HostCSR& R, const HostCSR& RA, const std::vector<double>& s);
+// G = [2S - S A S | (I - S A) P], S = diag(s): from a level's right-hand side and the coarse correction, stacked with
+// the latter from row `offset` on, to the post-smoothed iterate
+HostCSR folded_prolongation(const HostCSR& A, const HostCSR& P, const std::vector<double>& s, int offset);
 std::vector<double> dense_inverse(const HostCSR& A);  // row-major n x n; throws on singular
 
 }  // namespace mm

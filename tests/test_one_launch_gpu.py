@@ -81,6 +81,26 @@ def test_rows_dealt_out_over_every_number_of_lanes(cuda_ok, precision):
         assert np.array_equal(out[0][0], out[1][0])
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32_precond", "mixed"])
+@pytest.mark.parametrize("mesh", sorted(MESHES))
+def test_folded_levels_are_the_same_preconditioner(cuda_ok, mesh, precision):
+    """Prolongation and post-smoothing as one product against the two steps (without the fused restriction no level
+    is folded).  Both solves stop at 1e-12, so the potentials agree to that times the operator's condition
+    (~(box / h)^2 < 1e5)."""
+    s = _setup(MESHES[mesh])
+    prob = fem_utils.make_problem(s)
+    if precision != "fp64":
+        prob.set_precision(precision)
+    prob.build_poisson(1e-12, "amgcl")
+    m = syn.initial_state(s.N, seed=9, amplitude=0.3)
+    out = []
+    for restrict in (3, 0):
+        prob.set_option("fuse_restrict", restrict)
+        out.append(prob.solve_u(m, np.zeros(s.N), 1e-12))
+    assert out[0][3] == out[1][3] == 0 and abs(out[0][1] - out[1][1]) <= 1
+    assert np.abs(out[0][0] - out[1][0]).max() <= 1e-7 * np.abs(out[1][0]).max()
+
+
 def test_solves_in_flight_share_the_device_and_keep_their_bits(cuda_ok):
     """Several threads' solves: the number in flight changes how each runs, not what it returns."""
     s = _setup(MESHES["ragged"])
