@@ -12,8 +12,8 @@
 //    of one staged window: the descriptors differ only in their start address.  Halo outputs are
 //    computed and stored as zero, which keeps the padding invariant for the next layer.
 //  * Weight gradients reduce over voxels (K = voxels, M = input channels can be 16): they use
-//    warp-level mma.sync (m16n8k16, BF16 in, FP32 accumulate) with ldmatrix.trans staging, split
-//    over voxel ranges into per-block partials summed in a fixed order (deterministic).
+//    warp-level mma.sync (m16n8k16, BF16 in, FP32 accumulate) with ldmatrix.trans staging, nine taps
+//    a block, split over voxel ranges into per-block partials summed in a fixed order (deterministic).
 //  * Everything else (pooling, upsampling with skip addition, ReLU masks, the loss, Adam, the BF16
 //    weight copies, mesh <-> grid transfers) is plain elementwise CUDA.
 #include <cuda_bf16.h>
@@ -252,25 +252,23 @@ __global__ void __launch_bounds__(128) k_conv_tc(ConvArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// weight gradient (mma.sync m16n8k16, BF16 in, FP32 accumulate), split over voxel ranges
+// weight and bias gradients (mma.sync m16n8k16, BF16 in, FP32 accumulate), split over voxel ranges
 // ------------------------------------------------------------------------------------------------
 struct WgArgs {
   const uint4* x;   // layer input, cin / 8 chunk planes per sample
   const uint4* d;   // gradient of the pre-activation output, cout / 8 chunk planes per sample
-  float* part;      // [batch][nsplit][27][cin][cout]
+  float* part;      // [batch][nsplit]: [27][cin][cout], then cout bias gradients if `bias`
   Vol v;
   int cin, cout;
-  int vpb;          // voxels per block (multiple of 64)
+  int vpb;          // voxels per block
   int nsplit;
+  int bias;
 };
 
 __device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
                : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x2_t(uint32_t addr, uint32_t& r0, uint32_t& r1) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
 }
 __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                           uint32_t b0, uint32_t b1) {
@@ -281,113 +279,166 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+__device__ __forceinline__ void cp_async16(uint4* dst, const uint4* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(mtc::smem_u32(dst)), "l"(src) : "memory");
+}
+
+// A block takes the nine taps of one dz: it stages a tile of WG_TV voxels of d and the x rows that these taps
+// shift it to (one window: a tap's operand is its rows from dy P + dx on), and multiplies every tap from there.  A block
+// per tap read both from memory for each of the 27: 78 us a level-0 layer at 32^3, batch 8, and 24 us more for a pass
+// over d for the bias, which is summed here from the staged tile.  Warps: dy, and two halves of a tile's voxels; the
+// next tile's copies are in flight meanwhile.  What bounds it is the staging: 16 x 16 channels are three
+// multiplications for each four fragment loads.  A training pass at 32^3, batch 8: 2325 -> 1643 us; at 16^3, batch 1,
+// 1430 -> 1266; at 64^3, batch 2, 2869 -> 1892.
+constexpr int WG_TV = 128;
+constexpr int WG_THREADS = 192;
+__host__ __device__ inline int wg_window(int P) { return WG_TV + 2 * P + 2; }
 template <int CIT, int COT>
-__global__ void __launch_bounds__(128) k_wgrad(WgArgs a) {
-  constexpr int MTL = CIT / 16, NTL = COT / 8, TILES = MTL * NTL, TPW = (TILES + 3) / 4;
-  __shared__ __align__(16) uint4 Xs[CIT / 8][64];
-  __shared__ __align__(16) uint4 Ds[COT / 8][64];
+inline size_t wg_smem(int P) {
+  const size_t stages = 2 * ((size_t)(CIT / 8) * wg_window(P) + (size_t)(COT / 8) * WG_TV) * 16;
+  return std::max(stages, (size_t)9 * CIT * COT * 4);  // and the halves' sums
+}
+
+template <int CIT, int COT>
+__global__ void __launch_bounds__(WG_THREADS) k_wgrad(WgArgs a) {
+  constexpr int MTL = CIT / 16, NTL = COT / 8, XC = CIT / 8, DC = COT / 8;
+  extern __shared__ __align__(16) uint4 wg_sm[];
   const Vol v = a.v;
-  const int split = blockIdx.x;
+  const int P = v.P, XW = wg_window(P);
+  const size_t stage = (size_t)XC * XW + DC * WG_TV;
   int yy = blockIdx.y;
-  const int nct = a.cout / COT, nit = a.cin / CIT;
-  const int cot = yy % nct;
-  yy /= nct;
-  const int cit = yy % nit;
-  const int t = yy / nit;
-  const int b = blockIdx.z;
-  const int shift = (t / 9 - 1) * v.P * v.P + ((t / 3) % 3 - 1) * v.P + (t % 3 - 1);
+  const int dz = yy % 3;
+  yy /= 3;
+  const int nct = a.cout / COT;
+  const int cot = yy % nct, cit = yy / nct;
+  const int split = blockIdx.x, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float acc[TPW][4];
+  const int dy = warp % 3, half = warp / 3;
+  const int vbeg = v.t0 + split * a.vpb, vend = min(v.t1, vbeg + a.vpb);
+  const uint4* const xp = a.x + ((size_t)b * (a.cin / 8) + cit * XC) * v.plane + v.guard + (dz - 1) * P * P - (P + 1);
+  const uint4* const dp = a.d + ((size_t)b * (a.cout / 8) + cot * DC) * v.plane + v.guard;
+  // rows past the range are in x's guard; d's count as zero
+  auto load = [&](int v0, int st) {
+    uint4* const X = wg_sm + st * stage;
+    uint4* const D = X + (size_t)XC * XW;
 #pragma unroll
-  for (int q = 0; q < TPW; ++q)
+    for (int c = 0; c < XC; ++c)
+      for (int r = threadIdx.x; r < XW; r += WG_THREADS) cp_async16(X + c * XW + r, xp + (size_t)c * v.plane + v0 + r);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) acc[q][i] = 0.0f;
-  const int vbeg = v.t0 + split * a.vpb;
-  const int vend = min(v.t1, vbeg + a.vpb);
-  const size_t xp0 = (size_t)b * (a.cin / 8) + cit * (CIT / 8);
-  const size_t dp0 = (size_t)b * (a.cout / 8) + cot * (COT / 8);
-  for (int v0 = vbeg; v0 < vend; v0 += 64) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < (CIT / 8) * 64; i += 128) {
-      const int c = i >> 6, r = i & 63;
-      Xs[c][r] = a.x[(xp0 + c) * v.plane + v.guard + v0 + r + shift];
+    for (int c = 0; c < DC; ++c)
+      for (int r = threadIdx.x; r < WG_TV; r += WG_THREADS) {
+        if (v0 + r < vend) cp_async16(D + c * WG_TV + r, dp + (size_t)c * v.plane + v0 + r);
+        else D[c * WG_TV + r] = make_uint4(0, 0, 0, 0);
+      }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float acc[3][MTL * NTL][4];
+#pragma unroll
+  for (int t = 0; t < 3; ++t)
+#pragma unroll
+    for (int q = 0; q < MTL * NTL; ++q)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[t][q][i] = 0.0f;
+  const bool bias = a.bias && dz == 0 && cit == 0;
+  constexpr int BT = WG_THREADS / DC;  // threads of a chunk's bias sums
+  float bs[8] = {};
+  load(vbeg, 0);
+  int st = 0;
+  for (int v0 = vbeg; v0 < vend; v0 += WG_TV, st ^= 1) {
+    if (v0 + WG_TV < vend) {
+      load(v0 + WG_TV, st ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
-    for (int i = threadIdx.x; i < (COT / 8) * 64; i += 128) {
-      const int c = i >> 6, r = i & 63;
-      Ds[c][r] = (v0 + r < vend) ? a.d[(dp0 + c) * v.plane + v.guard + v0 + r] : make_uint4(0, 0, 0, 0);
-    }
     __syncthreads();
+    const uint4* const X = wg_sm + st * stage;
+    const uint4* const D = X + (size_t)XC * XW;
+#pragma unroll 1
+    for (int kk = half; kk < WG_TV / 16; kk += 2) {
+      const int mat = lane >> 3, r = lane & 7;
+      uint32_t bf[NTL][2];
 #pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
+      for (int ni = 0; ni < NTL; ni += 2)
+        ldsm_x4_t(mtc::smem_u32(D + (ni + (lane >> 4)) * WG_TV + kk * 16 + (lane & 15)), bf[ni][0], bf[ni][1],
+                  bf[ni + 1][0], bf[ni + 1][1]);
 #pragma unroll
-      for (int q = 0; q < TPW; ++q) {
-        const int j = warp + 4 * q;
-        if (j < TILES) {
-          const int mi = j / NTL, ni = j % NTL;
-          const int mat = lane >> 3, r = lane & 7;
-          const uint32_t aaddr = mtc::smem_u32(&Xs[mi * 2 + (mat & 1)][kk * 16 + (mat >> 1) * 8 + r]);
-          uint32_t a0, a1, a2, a3, b0, b1;
-          ldsm_x4_t(aaddr, a0, a1, a2, a3);
-          const int l16 = lane & 15;
-          const uint32_t baddr = mtc::smem_u32(&Ds[ni][kk * 16 + l16]);
-          ldsm_x2_t(baddr, b0, b1);
-          mma_16816(acc[q], a0, a1, a2, a3, b0, b1);
+      for (int t = 0; t < 3; ++t)
+#pragma unroll
+        for (int mi = 0; mi < MTL; ++mi) {
+          uint32_t a0, a1, a2, a3;
+          ldsm_x4_t(mtc::smem_u32(X + (mi * 2 + (mat & 1)) * XW + dy * P + t + kk * 16 + (mat >> 1) * 8 + r), a0, a1,
+                    a2, a3);
+#pragma unroll
+          for (int ni = 0; ni < NTL; ++ni) mma_16816(acc[t][mi * NTL + ni], a0, a1, a2, a3, bf[ni][0], bf[ni][1]);
         }
+    }
+    if (bias && threadIdx.x < BT * DC) {
+      for (int r = threadIdx.x % BT; r < WG_TV; r += BT) {
+        float f[8];
+        unpack8(D[threadIdx.x / BT * WG_TV + r], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) bs[j] += f[j];
       }
     }
+    __syncthreads();
   }
-  float* out = a.part + (((size_t)b * a.nsplit + split) * 27 + t) * (size_t)a.cin * a.cout;
+  // the halves' sums, then the block's partial
+  float* const sm = reinterpret_cast<float*>(wg_sm);
   const int g = lane >> 2, tg = lane & 3;
+  float* const out = a.part + ((size_t)b * a.nsplit + split) * ((size_t)27 * a.cin * a.cout + (a.bias ? a.cout : 0));
 #pragma unroll
-  for (int q = 0; q < TPW; ++q) {
-    const int j = warp + 4 * q;
-    if (j < TILES) {
-      const int mi = j / NTL, ni = j % NTL;
-      const int ci = cit * CIT + mi * 16 + g;
-      const int co = cot * COT + ni * 8 + 2 * tg;
-      out[(size_t)ci * a.cout + co] = acc[q][0];
-      out[(size_t)ci * a.cout + co + 1] = acc[q][1];
-      out[(size_t)(ci + 8) * a.cout + co] = acc[q][2];
-      out[(size_t)(ci + 8) * a.cout + co + 1] = acc[q][3];
+  for (int t = 0; t < 3; ++t)
+#pragma unroll
+    for (int q = 0; q < MTL * NTL; ++q) {
+      float4* const m = reinterpret_cast<float4*>(sm) + ((dy * 3 + t) * MTL * NTL + q) * 32 + lane;
+      if (half) *m = make_float4(acc[t][q][0], acc[t][q][1], acc[t][q][2], acc[t][q][3]);
     }
+  __syncthreads();
+  if (!half) {
+#pragma unroll
+    for (int t = 0; t < 3; ++t)
+#pragma unroll
+      for (int q = 0; q < MTL * NTL; ++q) {
+        const float4 o = reinterpret_cast<const float4*>(sm)[((dy * 3 + t) * MTL * NTL + q) * 32 + lane];
+        const int ci = cit * CIT + q / NTL * 16 + g, co = cot * COT + q % NTL * 8 + 2 * tg;
+        float* const w = out + ((size_t)((dz * 3 + dy) * 3 + t) * a.cin + ci) * a.cout + co;
+        *reinterpret_cast<float2*>(w) = make_float2(acc[t][q][0] + o.x, acc[t][q][1] + o.y);
+        *reinterpret_cast<float2*>(w + 8 * a.cout) = make_float2(acc[t][q][2] + o.z, acc[t][q][3] + o.w);
+      }
+  }
+  if (!bias) return;  // uniform
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) sm[threadIdx.x * 8 + j] = bs[j];
+  __syncthreads();
+  if (threadIdx.x < COT) {
+    float t = 0.0f;
+    for (int i = 0; i < BT; ++i) t += sm[(threadIdx.x / 8 * BT + i) * 8 + threadIdx.x % 8];
+    out[(size_t)27 * a.cin * a.cout + cot * COT + threadIdx.x] = t;
   }
 }
 
-// dW[i] = sum over (sample, split) of the partials, in order; rows ci >= keep_ci are zeroed
-__global__ void k_sum_parts(const float* part, int nparts, int n, int cin, int cout, int keep_ci, float* dst) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int k = 0; k < nparts; ++k) s += part[(size_t)k * n + i];
-    const int ci = (i / cout) % cin;
-    dst[i] = ci < keep_ci ? (float)s : 0.0f;
+// The gradients from the partials (weights, then biases if any), in FP64 and a fixed order: eight threads of a block
+// take every eighth partial of an element each.  Rows ci >= keep_ci of the weights are zeroed.  One thread an element
+// waited for its partials' loads and FP64 adds in turn: 12-18 us whatever the size.
+__global__ void __launch_bounds__(256) k_sum_parts(const float* part, int nparts, int nw, int n, int cin, int cout,
+                                                   int keep_ci, float* dw, float* db) {
+  __shared__ double s[8][32];
+  const int lane = threadIdx.x & 31, j = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  double t = 0.0;
+  if (i < n) {
+#pragma unroll 4
+    for (int k = j; k < nparts; k += 8) t += part[(size_t)k * n + i];
   }
-}
-
-// bias-gradient partials: bpart[(b * nsplit + split) * cout + co] = sum over the split's voxels
-__global__ void __launch_bounds__(128) k_bias_part(const uint4* d, Vol v, int cout, int vpb, int nsplit, float* bpart) {
-  __shared__ float s[128][8];
-  const int split = blockIdx.x, b = blockIdx.y;
-  const int nch = cout / 8;
-  const int vbeg = v.t0 + split * vpb, vend = min(v.t1, vbeg + vpb);
-  for (int c = 0; c < nch; ++c) {
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    const uint4* pl = d + ((size_t)b * nch + c) * v.plane + v.guard;
-    for (int p = vbeg + threadIdx.x; p < vend; p += 128) {
-      float f[8];
-      unpack8(pl[p], f);
+  s[j][lane] = t;
+  __syncthreads();
+  if (j || i >= n) return;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += f[j];
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) s[threadIdx.x][j] = acc[j];
-    __syncthreads();
-    if (threadIdx.x < 8) {
-      float t = 0.0f;
-      for (int i = 0; i < 128; ++i) t += s[i][threadIdx.x];
-      bpart[((size_t)b * nsplit + split) * cout + c * 8 + threadIdx.x] = t;
-    }
-    __syncthreads();
-  }
+  for (int k = 1; k < 8; ++k) t += s[k][lane];
+  if (i >= nw) db[i - nw] = (float)t;
+  else dw[i] = (i / cout) % cin < keep_ci ? (float)t : 0.0f;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -700,7 +751,8 @@ constexpr int IN_CH = 4;
 constexpr int NSPLIT_MAX = 64;
 
 inline int nt_of(int cout) { return std::min(cout, 64); }
-inline int cit_of(int cin) { return std::min(cin, 64); }
+// channels of a block of the weight gradient: 3 x 32 x 32 sums are 96 registers a thread
+inline int wg_of(int c) { return std::min(c, 32); }
 
 template <class F>
 void conv_dispatch(int cin, int nt, F&& f) {
@@ -716,14 +768,13 @@ void conv_dispatch(int cin, int nt, F&& f) {
 }
 
 template <class F>
-void wgrad_dispatch(int cit, int cot, F&& f) {
-#define WG_CASE(A, B)                   \
-  if (cit == A && cot == B) {           \
-    f(mmn::k_wgrad<A, B>);              \
-    return;                             \
+void wgrad_dispatch(int cit, int cot, int P, F&& f) {
+#define WG_CASE(A, B)                                \
+  if (cit == A && cot == B) {                        \
+    f(mmn::k_wgrad<A, B>, mmn::wg_smem<A, B>(P));    \
+    return;                                          \
   }
-  WG_CASE(16, 16) WG_CASE(16, 32) WG_CASE(16, 64) WG_CASE(32, 16) WG_CASE(32, 32) WG_CASE(32, 64) WG_CASE(64, 16)
-  WG_CASE(64, 32) WG_CASE(64, 64)
+  WG_CASE(16, 16) WG_CASE(16, 32) WG_CASE(32, 16) WG_CASE(32, 32)
 #undef WG_CASE
   throw UFail{MM_ERR_ARG, "unsupported weight-gradient shape"};
 }
@@ -753,7 +804,6 @@ struct mm_unet {
   uint4* dT[T_COUNT] = {};
   float* part = nullptr;
   size_t part_cap = 0;
-  float* bpart = nullptr;
   double* lpart = nullptr;
   double* h_lpart = nullptr;
   float* stage_in = nullptr;   // FP32 [B][G^3][4]
@@ -763,7 +813,7 @@ struct mm_unet {
   cudaGraphExec_t fwd_exec[8] = {};   // captured forward passes (batch sizes 1..8), on the in-place input
   bool fwd_warm = false;              // one forward has run (kernel attributes set) before any capture
   cudaEvent_t ev_after = nullptr;     // ordering point taken on a caller's stream (mm_unet_predict_dev)
-  std::vector<std::pair<const void*, size_t>> attr_done;
+  std::vector<const void*> attr_done;  // kernels allowed all of an SM's shared memory
   bool train_bias = true;      // false: bias gradients are zero (biases stay as set)
 
   template <class T>
@@ -795,6 +845,13 @@ struct mm_unet {
     if (e) throw UFail{MM_ERR_CUDA, "a tensor-core convolution gave up waiting for its operands or accumulators"};
   }
 
+  // The limit belongs to the kernel, not to this network: one for every size, so that no network lowers another's.
+  void allow_smem(const void* kern) {
+    if (std::find(attr_done.begin(), attr_done.end(), kern) != attr_done.end()) return;
+    UCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    attr_done.push_back(kern);
+  }
+
   void conv(int l, const uint4* in, uint4* out, int nb, bool transposed) {
     const LayerDef& d = DEFS[l];
     const int cin = transposed ? d.cout : d.cin;
@@ -815,34 +872,22 @@ struct mm_unet {
     const size_t smem = mmn::conv_smem(v.P, cin, nt);
     dim3 grid((unsigned)((v.t1 - v.t0 + 128 * mmn::MT - 1) / (128 * mmn::MT)), (unsigned)(cout / nt), (unsigned)nb);
     conv_dispatch(cin, nt, [&](auto kern) {
-      // the kernel's shared-memory limit only ever grows (and is not touched during a graph capture
-      // once every size has been seen)
-      size_t* cur = nullptr;
-      for (auto& kv : attr_done)
-        if (kv.first == (const void*)kern) cur = &kv.second;
-      if (!cur) {
-        attr_done.emplace_back((const void*)kern, 0);
-        cur = &attr_done.back().second;
-      }
-      if (smem > *cur) {
-        UCK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        *cur = smem;
-      }
+      allow_smem((const void*)kern);
       kern<<<grid, 128, smem, st>>>(a);
       UCK(cudaGetLastError());
     });
   }
 
-  // voxels per block and splits of the weight-gradient reduction of a layer
+  // voxels per block and splits of the weight-gradient reduction of a layer: three blocks an SM
   void wg_split(int l, int nb, int& vpb, int& ns) const {
     const LayerDef& d = DEFS[l];
     const mmn::Vol& v = vol[d.level];
-    const int range = v.t1 - v.t0;
-    const int tiles = 27 * (d.cin / cit_of(d.cin)) * (d.cout / nt_of(d.cout));
-    ns = std::max(1, std::min(NSPLIT_MAX, 2048 / std::max(1, tiles * nb)));
-    ns = std::min(ns, (range + 63) / 64);
-    vpb = ((range + ns - 1) / ns + 63) / 64 * 64;
-    ns = (range + vpb - 1) / vpb;
+    const int range = v.t1 - v.t0, tiles = (range + mmn::WG_TV - 1) / mmn::WG_TV;
+    const int blocks = 3 * (d.cin / wg_of(d.cin)) * (d.cout / wg_of(d.cout)) * nb;
+    ns = std::max(1, std::min({NSPLIT_MAX, tiles, 456 / blocks}));
+    const int per = (tiles + ns - 1) / ns;
+    vpb = per * mmn::WG_TV;
+    ns = (tiles + per - 1) / per;
   }
 
   void bwd_layer(int l, uint4* dy, const uint4* x, const uint4* y, uint4* dx, int nb) {
@@ -864,24 +909,19 @@ struct mm_unet {
     a.cout = d.cout;
     a.vpb = vpb;
     a.nsplit = ns;
-    const int cit = cit_of(d.cin), cot = nt_of(d.cout);
-    dim3 grid((unsigned)ns, (unsigned)(27 * (d.cin / cit) * (d.cout / cot)), (unsigned)nb);
-    wgrad_dispatch(cit, cot, [&](auto kern) {
-      kern<<<grid, 128, 0, st>>>(a);
+    a.bias = train_bias ? 1 : 0;
+    const int cit = wg_of(d.cin), cot = wg_of(d.cout);
+    dim3 grid((unsigned)ns, (unsigned)(3 * (d.cin / cit) * (d.cout / cot)), (unsigned)nb);
+    wgrad_dispatch(cit, cot, v.P, [&](auto kern, size_t smem) {
+      allow_smem((const void*)kern);
+      kern<<<grid, mmn::WG_THREADS, smem, st>>>(a);
       UCK(cudaGetLastError());
     });
-    const int nw = 27 * d.cin * d.cout;
-    mmn::k_sum_parts<<<grid1d(nw), 256, 0, st>>>(part, nb * ns, nw, d.cin, d.cout, l == L_E0A ? IN_CH : d.cin,
-                                                 g + woff[l]);
+    const int nw = 27 * d.cin * d.cout, n = nw + (train_bias ? d.cout : 0);
+    mmn::k_sum_parts<<<(n + 31) / 32, 256, 0, st>>>(part, nb * ns, nw, n, d.cin, d.cout, l == L_E0A ? IN_CH : d.cin,
+                                                    g + woff[l], g + boff[l]);
     UCK(cudaGetLastError());
-    if (train_bias) {
-      mmn::k_bias_part<<<dim3((unsigned)ns, (unsigned)nb), 128, 0, st>>>(dy, v, d.cout, vpb, ns, bpart);
-      UCK(cudaGetLastError());
-      mmn::k_sum_parts<<<grid1d(d.cout), 256, 0, st>>>(bpart, nb * ns, d.cout, 1, d.cout, 1, g + boff[l]);
-      UCK(cudaGetLastError());
-    } else {
-      UCK(cudaMemsetAsync(g + boff[l], 0, d.cout * sizeof(float), st));
-    }
+    if (!train_bias) UCK(cudaMemsetAsync(g + boff[l], 0, d.cout * sizeof(float), st));
     if (dx) conv(l, dy, dx, nb, true);
   }
 
@@ -1055,21 +1095,15 @@ int mm_unet_create(int grid, int batch, mm_unet** out) {
       u->T[t] = u->tensor(TDEF[t][0], TDEF[t][1]);
       u->dT[t] = u->tensor(TDEF[t][0], TDEF[t][1]);
     }
-    size_t cap = 0, bcap = 0;
-    for (int l = 0; l < MM_UNET_LAYERS; ++l) {
-      int vpb = 0, ns = 0;
-      u->wg_split(l, batch, vpb, ns);
-      cap = std::max(cap, (size_t)batch * ns * 27 * DEFS[l].cin * DEFS[l].cout);
-      bcap = std::max(bcap, (size_t)batch * ns * DEFS[l].cout);
-      for (int nb = 1; nb < batch; ++nb) {  // smaller batches split further
+    size_t cap = 0;
+    for (int l = 0; l < MM_UNET_LAYERS; ++l)
+      for (int nb = 1; nb <= batch; ++nb) {  // smaller batches split further
+        int vpb = 0, ns = 0;
         u->wg_split(l, nb, vpb, ns);
-        cap = std::max(cap, (size_t)nb * ns * 27 * DEFS[l].cin * DEFS[l].cout);
-        bcap = std::max(bcap, (size_t)nb * ns * DEFS[l].cout);
+        cap = std::max(cap, (size_t)nb * ns * ((size_t)27 * DEFS[l].cin + 1) * DEFS[l].cout);
       }
-    }
     u->part = u->alloc<float>(cap);
     u->part_cap = cap;
-    u->bpart = u->alloc<float>(bcap);
     u->lpart = u->alloc<double>(256);
     UCK(cudaMallocHost(&u->h_lpart, 256 * sizeof(double)));
     const size_t nv = (size_t)batch * grid * grid * grid;
