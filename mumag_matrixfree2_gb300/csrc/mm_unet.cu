@@ -419,26 +419,39 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad(WgArgs a) {
   }
 }
 
-// The gradients from the partials (weights, then biases if any), in FP64 and a fixed order: eight threads of a block
-// take every eighth partial of an element each.  Rows ci >= keep_ci of the weights are zeroed.  One thread an element
-// waited for its partials' loads and FP64 adds in turn: 12-18 us whatever the size.
-__global__ void __launch_bounds__(256) k_sum_parts(const float* part, int nparts, int nw, int n, int cin, int cout,
-                                                   int keep_ci, float* dw, float* db) {
-  __shared__ double s[8][32];
-  const int lane = threadIdx.x & 31, j = threadIdx.x >> 5;
-  const int i = blockIdx.x * 32 + lane;
-  double t = 0.0;
+// (h, l) += v exactly up to the rounding of l
+__device__ __forceinline__ void sum2(float& h, float& l, float v) {
+  const float t = h + v, z = t - h;
+  l += (h - (t - z)) + (v - z);
+  h = t;
+}
+
+// The gradients from the partials (weights, then biases if any) in a fixed order: 2^lg threads of a block take every
+// 2^lg-th partial of an element each.  Rows ci >= keep_ci of the weights are zeroed.  The sums are FP32 pairs (a sum and
+// its rounding errors, ~2^-47): conversions and adds of FP64 sums held the FP64 pipe for 10-30 us a layer.
+__global__ void __launch_bounds__(256) k_sum_parts(const float* part, int nparts, int lg, int nw, int n, int cin,
+                                                   int cout, int keep_ci, float* dw, float* db) {
+  __shared__ float2 s[256];
+  const int per = 256 >> lg, j = threadIdx.x / per;
+  const int i = blockIdx.x * per + threadIdx.x % per;
+  float h = 0.0f, l = 0.0f;
   if (i < n) {
-#pragma unroll 4
-    for (int k = j; k < nparts; k += 8) t += part[(size_t)k * n + i];
+#pragma unroll 8
+    for (int k = j; k < nparts; k += 1 << lg) sum2(h, l, part[(size_t)k * n + i]);
   }
-  s[j][lane] = t;
-  __syncthreads();
-  if (j || i >= n) return;
-#pragma unroll
-  for (int k = 1; k < 8; ++k) t += s[k][lane];
-  if (i >= nw) db[i - nw] = (float)t;
-  else dw[i] = (i / cout) % cin < keep_ci ? (float)t : 0.0f;
+  if (lg) {
+    s[threadIdx.x] = make_float2(h, l);
+    __syncthreads();
+    if (j) return;
+    for (int k = 1; k < 1 << lg; ++k) {
+      const float2 o = s[threadIdx.x + k * per];
+      sum2(h, l, o.x);
+      l += o.y;
+    }
+  }
+  if (i >= n) return;
+  if (i >= nw) db[i - nw] = h + l;
+  else dw[i] = (i / cout) % cin < keep_ci ? h + l : 0.0f;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -918,8 +931,10 @@ struct mm_unet {
       UCK(cudaGetLastError());
     });
     const int nw = 27 * d.cin * d.cout, n = nw + (train_bias ? d.cout : 0);
-    mmn::k_sum_parts<<<(n + 31) / 32, 256, 0, st>>>(part, nb * ns, nw, n, d.cin, d.cout, l == L_E0A ? IN_CH : d.cin,
-                                                    g + woff[l], g + boff[l]);
+    int lg = 0;  // threads an element (log2): two blocks an SM
+    while (lg < 3 && (n << lg) < 304 * 256 && 2 << lg <= nb * ns) ++lg;
+    mmn::k_sum_parts<<<((n << lg) + 255) / 256, 256, 0, st>>>(part, nb * ns, lg, nw, n, d.cin, d.cout,
+                                                              l == L_E0A ? IN_CH : d.cin, g + woff[l], g + boff[l]);
     UCK(cudaGetLastError());
     if (!train_bias) UCK(cudaMemsetAsync(g + boff[l], 0, d.cout * sizeof(float), st));
     if (dx) conv(l, dy, dx, nb, true);
