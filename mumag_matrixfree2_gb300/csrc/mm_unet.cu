@@ -91,29 +91,31 @@ struct ConvArgs {
   Vol v;
   int cin, cout;
   int relu;
+  int nst;           // stage buffers
   int* err;          // set to 1 when a wait gave up
 };
 
 // Shared memory of one CTA: barriers, then NST stages of A windows (3 dz x 2 chunks x WL rows) and
-// B weights (27 taps x 2 chunks x NT rows), 16 bytes per row.
+// B weights (27 taps x 2 chunks x NT rows), 16 bytes per row.  As many stages as fit, up to four: with two, a coarse
+// level's few CTAs waited for the copies of every second stage.
 __host__ __device__ inline int conv_wl(int P) { return 128 * MT + 2 * P + 2; }
-__host__ __device__ inline size_t conv_smem(int P, int cin, int NT) {
-  const int nst = cin >= 32 ? 2 : 1;
-  return 1024 + (size_t)nst * ((size_t)6 * conv_wl(P) * 16 + (size_t)54 * NT * 16);
+constexpr int CONV_STAGES = 4;
+inline size_t conv_stage(int P, int NT) { return (size_t)6 * conv_wl(P) * 16 + (size_t)54 * NT * 16; }
+inline int conv_stages(int P, int cin, int NT, int most) {
+  return (int)std::min<size_t>({(size_t)most, (size_t)cin / 16, (size_t)(226 * 1024) / conv_stage(P, NT)});
 }
 
 template <int CIN, int NT>
 __global__ void __launch_bounds__(128) k_conv_tc(ConvArgs a) {
   constexpr int NCP = CIN / 16;           // K stages: 16 input channels each
-  constexpr int NST = NCP >= 2 ? 2 : 1;   // stage buffers
   constexpr uint32_t NCOL = (MT * NT <= 32) ? 32 : (MT * NT <= 64 ? 64 : (MT * NT <= 128 ? 128 : 256));
   extern __shared__ __align__(1024) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);      // [NST]
-  uint64_t* done = full + 2;                                // [NST]
+  uint64_t* done = full + CONV_STAGES;                      // [NST]
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + 64);
   int* s_fail = reinterpret_cast<int*>(smem + 68);
   const Vol v = a.v;
-  const int P = v.P;
+  const int P = v.P, NST = a.nst;
   const int WL = conv_wl(P);
   unsigned char* Abuf = smem + 1024;
   const size_t Astage = (size_t)6 * WL * 16;
@@ -156,10 +158,9 @@ __global__ void __launch_bounds__(128) k_conv_tc(ConvArgs a) {
         }
       mtc::bulk_g2s(B, a.wk + ((size_t)cot * NCP + cp) * 54 * NT, (uint32_t)Bstage, &full[st]);
     };
-    // bookkeeping for the failure path: chunks whose copies were issued / seen complete, the last
-    // chunk whose MMAs were committed and whether their completion was seen
+    // bookkeeping for the failure path: chunks whose copies were issued / seen complete, and the last
+    // chunk whose MMAs were committed
     int issued = 0, loaded = 0, committed = -1;
-    bool mma_seen = true;
     for (int s = 0; s < NST && s < NCP; ++s, ++issued) issue(s, s);
     constexpr uint32_t IDESC = mtc::idesc_bf16(128, NT);
     bool ok = true;
@@ -172,29 +173,28 @@ __global__ void __launch_bounds__(128) k_conv_tc(ConvArgs a) {
       }
       loaded = cp + 1;
       mtc::tc_fence_after();
-      const uint32_t As = mtc::smem_u32(Abuf + st * Astage);
-      const uint32_t Bs = mtc::smem_u32(Bbuf + st * Bstage);
+      // a descriptor's address counts rows of 16 bytes: a tap's is the window's plus its rows
+      const uint64_t ad = mtc::sdesc(mtc::smem_u32(Abuf + st * Astage), (uint32_t)WL * 16, 128);
+      const uint64_t bd = mtc::sdesc(mtc::smem_u32(Bbuf + st * Bstage), NT * 16, 128);
 #pragma unroll 1
-      for (int t = 0; t < 27; ++t) {
-        const int dz = t / 9, dy = (t / 3) % 3, dx = t % 3;  // shifts + 1
-        const uint64_t bd = mtc::sdesc(Bs + (uint32_t)(t * 2 * NT * 16), NT * 16, 128);
+      for (int q = 0; q < 9; ++q) {
+        const int row = (q / 3) * 2 * WL + (q % 3) * P;  // dz, dy shifts
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          const uint32_t aoff = (uint32_t)((dz * 2 * WL + mt * 128 + dy * P + dx) * 16);
-          const uint64_t ad = mtc::sdesc(As + aoff, (uint32_t)WL * 16, 128);
-          mtc::mma_bf16(tbase + (uint32_t)(mt * NT), ad, bd, IDESC, cp > 0 || t > 0);
-        }
+        for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt)
+            mtc::mma_bf16(tbase + (uint32_t)(mt * NT), ad + (uint32_t)(row + dx + mt * 128),
+                          bd + (uint32_t)((q * 3 + dx) * 2 * NT), IDESC, cp > 0 || q > 0 || dx > 0);
       }
       mtc::mma_commit(&done[st]);
       committed = cp;
-      mma_seen = false;
-      if (cp + NST < NCP) {
-        if (!mtc::mbar_wait(&done[st], par)) {
+      // the chunk before this one gives its stage to the next copies, while this one's MMAs run
+      if (cp > 0 && issued < NCP) {
+        if (!mtc::mbar_wait(&done[(cp - 1) % NST], (uint32_t)((cp - 1) / NST) & 1u)) {
           ok = false;
           break;
         }
-        mma_seen = true;  // a commit's arrival covers every earlier MMA of this thread
-        issue(cp + NST, st);
+        issue(issued, (cp - 1) % NST);
         ++issued;
       }
     }
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(128) k_conv_tc(ConvArgs a) {
       // every later call of the network, an error.
       *s_fail = 1;
       atomicExch(a.err, 1);
-      if (committed >= 0 && !mma_seen) mtc::mbar_wait(&done[committed % NST], (uint32_t)(committed / NST) & 1u);
+      if (committed >= 0) mtc::mbar_wait(&done[committed % NST], (uint32_t)(committed / NST) & 1u);
       for (int c = loaded; c < issued; ++c) mtc::mbar_wait(&full[c % NST], (uint32_t)(c / NST) & 1u);
     }
   }
@@ -882,8 +882,10 @@ struct mm_unet {
     a.cout = cout;
     a.relu = (!transposed && d.relu) ? 1 : 0;
     a.err = d_err;
-    const size_t smem = mmn::conv_smem(v.P, cin, nt);
     dim3 grid((unsigned)((v.t1 - v.t0 + 128 * mmn::MT - 1) / (128 * mmn::MT)), (unsigned)(cout / nt), (unsigned)nb);
+    // more CTAs than SMs share them, and hide each other's copies
+    a.nst = mmn::conv_stages(v.P, cin, nt, grid.x * grid.y * grid.z <= 152 ? mmn::CONV_STAGES : 2);
+    const size_t smem = 1024 + a.nst * mmn::conv_stage(v.P, nt);
     conv_dispatch(cin, nt, [&](auto kern) {
       allow_smem((const void*)kern);
       kern<<<grid, 128, smem, st>>>(a);
