@@ -87,6 +87,7 @@ struct ConvArgs {
   const uint4* in;   // input activations, cin / 8 chunk planes per sample
   const uint4* wk;   // weights [cout/NT][cin/16][27][2][NT][8] bf16
   const float* bias; // cout, or null
+  const uint4* mask; // null, or the activations of the layer before (out's planes): out = 0 where they are 0
   uint4* out;        // output activations, cout / 8 chunk planes per sample
   Vol v;
   int cin, cout;
@@ -234,14 +235,24 @@ __global__ void __launch_bounds__(128) k_conv_tc(ConvArgs a) {
             if (a.relu) y = fmaxf(y, 0.0f);
             acc[j] = in ? y : 0.0f;
           }
+          const size_t at = (out_plane0 + co0 / 8) * v.plane + v.guard + p;
+          if (a.mask) {
+            float m[8];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              unpack8(a.mask[at + (size_t)h * v.plane], m);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) acc[8 * h + j] = m[j] > 0.0f ? acc[8 * h + j] : 0.0f;
+            }
+          }
           float lo[8], hi[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             lo[j] = acc[j];
             hi[j] = acc[8 + j];
           }
-          a.out[(out_plane0 + co0 / 8) * v.plane + v.guard + p] = pack8(lo);
-          a.out[(out_plane0 + co0 / 8 + 1) * v.plane + v.guard + p] = pack8(hi);
+          a.out[at] = pack8(lo);
+          a.out[at + v.plane] = pack8(hi);
         }
       }
     }
@@ -457,6 +468,14 @@ __global__ void __launch_bounds__(256) k_sum_parts(const float* part, int nparts
 // ------------------------------------------------------------------------------------------------
 // elementwise kernels (one thread per interior voxel and 8-channel chunk)
 // ------------------------------------------------------------------------------------------------
+// zero where the activations y of a ReLU are zero
+__device__ __forceinline__ void masked(float (&d)[8], const uint4& y) {
+  float m[8];
+  unpack8(y, m);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) d[j] = m[j] > 0.0f ? d[j] : 0.0f;
+}
+
 // out (level G/2) = 2x2x2 average of in (level G)
 __global__ void k_pool(const uint4* in, Vol vf, uint4* out, Vol vc, int nch, int nb) {
   const int Gc = vc.G;
@@ -501,7 +520,8 @@ __global__ void k_up_add(const uint4* in, Vol vc, const uint4* skip, uint4* out,
 }
 
 // d_fine = d_coarse(parent) / 8 + d_skip
-__global__ void k_pool_bwd_add(const uint4* dc, Vol vc, const uint4* dskip, uint4* df, Vol vf, int nch, int nb) {
+__global__ void k_pool_bwd_add(const uint4* dc, Vol vc, const uint4* dskip, const uint4* mask, uint4* df, Vol vf, int nch,
+                               int nb) {
   const int G = vf.G;
   const long long n = (long long)nb * nch * G * G * G;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -516,12 +536,13 @@ __global__ void k_pool_bwd_add(const uint4* dc, Vol vc, const uint4* dskip, uint
     unpack8(dskip[pl * vf.plane + vf.guard + pf], s);
 #pragma unroll
     for (int j = 0; j < 8; ++j) a[j] = a[j] * 0.125f + s[j];
+    masked(a, mask[pl * vf.plane + vf.guard + pf]);
     df[pl * vf.plane + vf.guard + pf] = pack8(a);
   }
 }
 
 // d_coarse = sum of the 8 children of d_fine
-__global__ void k_up_bwd(const uint4* df, Vol vf, uint4* dc, Vol vc, int nch, int nb) {
+__global__ void k_up_bwd(const uint4* df, Vol vf, const uint4* mask, uint4* dc, Vol vc, int nch, int nb) {
   const int Gc = vc.G;
   const long long n = (long long)nb * nch * Gc * Gc * Gc;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -537,28 +558,12 @@ __global__ void k_up_bwd(const uint4* df, Vol vf, uint4* dc, Vol vc, int nch, in
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] += f[j];
     }
-    dc[pl * vc.plane + vc.guard + flat(vc, z, y, x)] = pack8(acc);
+    const size_t at = pl * vc.plane + vc.guard + flat(vc, z, y, x);
+    masked(acc, mask[at]);
+    dc[at] = pack8(acc);
   }
 }
 
-// d <- d * (y > 0) (ReLU backward, in place)
-__global__ void k_relu_mask(uint4* d, const uint4* y, Vol v, int nch, int nb) {
-  const int G = v.G;
-  const long long n = (long long)nb * nch * G * G * G;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    long long r = i;
-    const int x = r % G; r /= G;
-    const int yy = r % G; r /= G;
-    const int z = r % G; r /= G;
-    const size_t at = (size_t)r * v.plane + v.guard + flat(v, z, yy, x);
-    float a[8], m[8];
-    unpack8(d[at], a);
-    unpack8(y[at], m);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) a[j] = m[j] > 0.0f ? a[j] : 0.0f;
-    d[at] = pack8(a);
-  }
-}
 
 // FP32 [nb][G^3][4] -> chunk 0 of the input tensor (channels 4..7 zero; chunk 1 stays zero)
 __global__ void k_pack_input(const float* src, Vol v, uint4* x, int nb) {
@@ -825,6 +830,8 @@ struct mm_unet {
   int nb_fwd = 0;              // samples of the last forward
   cudaGraphExec_t fwd_exec[8] = {};   // captured forward passes (batch sizes 1..8), on the in-place input
   bool fwd_warm = false;              // one forward has run (kernel attributes set) before any capture
+  cudaStream_t st_w = nullptr;  // the weights' gradients of a backward pass
+  cudaEvent_t ev_dy = nullptr, ev_dw = nullptr;  // a layer's dy is ready; the weights' gradients are
   cudaEvent_t ev_after = nullptr;     // ordering point taken on a caller's stream (mm_unet_predict_dev)
   std::vector<const void*> attr_done;  // kernels allowed all of an SM's shared memory
   bool train_bias = true;      // false: bias gradients are zero (biases stay as set)
@@ -865,7 +872,7 @@ struct mm_unet {
     attr_done.push_back(kern);
   }
 
-  void conv(int l, const uint4* in, uint4* out, int nb, bool transposed) {
+  void conv(int l, const uint4* in, uint4* out, int nb, bool transposed, const uint4* mask = nullptr) {
     const LayerDef& d = DEFS[l];
     const int cin = transposed ? d.cout : d.cin;
     const int cout = transposed ? d.cin : d.cout;
@@ -876,6 +883,7 @@ struct mm_unet {
     a.in = in;
     a.wk = transposed ? wkT[l] : (n16 ? wk16[l] : wk[l]);
     a.bias = transposed ? nullptr : p + boff[l];
+    a.mask = mask;
     a.out = out;
     a.v = v;
     a.cin = cin;
@@ -905,14 +913,15 @@ struct mm_unet {
     ns = (tiles + per - 1) / per;
   }
 
-  void bwd_layer(int l, uint4* dy, const uint4* x, const uint4* y, uint4* dx, int nb) {
+  // The gradients of a layer from dy, that of its output before the ReLU (its producer masked it), and dx if asked for,
+  // masked by the ReLU (`mask`, may be null) that its input came from.  Only dx is waited for by the layers before, so
+  // the weights' run beside it on a stream of their own, which backward() joins.
+  void bwd_layer(int l, const uint4* dy, const uint4* x, uint4* dx, const uint4* mask, int nb) {
     const LayerDef& d = DEFS[l];
     const mmn::Vol& v = vol[d.level];
-    if (d.relu) {
-      const long long n = (long long)nb * (d.cout / 8) * v.G * v.G * v.G;
-      mmn::k_relu_mask<<<grid1d(n), 256, 0, st>>>(dy, y, v, d.cout / 8, nb);
-      UCK(cudaGetLastError());
-    }
+    UCK(cudaEventRecord(ev_dy, st));
+    UCK(cudaStreamWaitEvent(st_w, ev_dy, 0));
+    if (dx) conv(l, dy, dx, nb, true, mask);
     int vpb = 0, ns = 0;
     wg_split(l, nb, vpb, ns);
     mmn::WgArgs a{};
@@ -929,17 +938,16 @@ struct mm_unet {
     dim3 grid((unsigned)ns, (unsigned)(3 * (d.cin / cit) * (d.cout / cot)), (unsigned)nb);
     wgrad_dispatch(cit, cot, v.P, [&](auto kern, size_t smem) {
       allow_smem((const void*)kern);
-      kern<<<grid, mmn::WG_THREADS, smem, st>>>(a);
+      kern<<<grid, mmn::WG_THREADS, smem, st_w>>>(a);
       UCK(cudaGetLastError());
     });
     const int nw = 27 * d.cin * d.cout, n = nw + (train_bias ? d.cout : 0);
     int lg = 0;  // threads an element (log2): two blocks an SM
     while (lg < 3 && (n << lg) < 304 * 256 && 2 << lg <= nb * ns) ++lg;
-    mmn::k_sum_parts<<<((n << lg) + 255) / 256, 256, 0, st>>>(part, nb * ns, lg, nw, n, d.cin, d.cout,
+    mmn::k_sum_parts<<<((n << lg) + 255) / 256, 256, 0, st_w>>>(part, nb * ns, lg, nw, n, d.cin, d.cout,
                                                               l == L_E0A ? IN_CH : d.cin, g + woff[l], g + boff[l]);
     UCK(cudaGetLastError());
-    if (!train_bias) UCK(cudaMemsetAsync(g + boff[l], 0, d.cout * sizeof(float), st));
-    if (dx) conv(l, dy, dx, nb, true);
+    if (!train_bias) UCK(cudaMemsetAsync(g + boff[l], 0, d.cout * sizeof(float), st_w));
   }
 
   void prep_weights() {
@@ -971,17 +979,17 @@ struct mm_unet {
                                                                                    nch, nb);
     UCK(cudaGetLastError());
   }
-  void up_bwd(int tf, int tc, int nb) {  // dT[tc] = sum of children of dT[tf]
+  void up_bwd(int tf, int tc, int nb) {  // dT[tc] = sum of children of dT[tf], masked
     const mmn::Vol &vf = vol[TDEF[tf][0]], &vc = vol[TDEF[tc][0]];
     const int nch = TDEF[tc][1] / 8;
-    mmn::k_up_bwd<<<grid1d((long long)nb * nch * vc.G * vc.G * vc.G), 256, 0, st>>>(dT[tf], vf, dT[tc], vc, nch, nb);
+    mmn::k_up_bwd<<<grid1d((long long)nb * nch * vc.G * vc.G * vc.G), 256, 0, st>>>(dT[tf], vf, T[tc], dT[tc], vc, nch, nb);
     UCK(cudaGetLastError());
   }
-  void pool_bwd_add(int tc, int tskip, int tf, int nb) {  // dT[tf] = dT[tc]/8 + dT[tskip]
+  void pool_bwd_add(int tc, int tskip, int tf, int nb) {  // dT[tf] = dT[tc]/8 + dT[tskip], masked
     const mmn::Vol &vc = vol[TDEF[tc][0]], &vf = vol[TDEF[tf][0]];
     const int nch = TDEF[tf][1] / 8;
     mmn::k_pool_bwd_add<<<grid1d((long long)nb * nch * vf.G * vf.G * vf.G), 256, 0, st>>>(dT[tc], vc, dT[tskip],
-                                                                                         dT[tf], vf, nch, nb);
+                                                                                         T[tf], dT[tf], vf, nch, nb);
     UCK(cudaGetLastError());
   }
 
@@ -1017,27 +1025,29 @@ struct mm_unet {
     mmn::k_loss<<<256, 256, 0, st>>>(T[T_OUT], v0, 2, d_target, nb, dT[T_OUT], lpart);
     UCK(cudaGetLastError());
     UCK(cudaMemcpyAsync(h_lpart, lpart, 256 * sizeof(double), cudaMemcpyDeviceToHost, st));
-    bwd_layer(L_D0B, dT[T_OUT], T[T_YD0A], T[T_OUT], dT[T_YD0A], nb);
-    bwd_layer(L_D0A, dT[T_YD0A], T[T_H0], T[T_YD0A], dT[T_H0], nb);
+    bwd_layer(L_D0B, dT[T_OUT], T[T_YD0A], dT[T_YD0A], T[T_YD0A], nb);
+    bwd_layer(L_D0A, dT[T_YD0A], T[T_H0], dT[T_H0], nullptr, nb);
     up_bwd(T_H0, T_YD1B, nb);
-    bwd_layer(L_D1B, dT[T_YD1B], T[T_YD1A], T[T_YD1B], dT[T_YD1A], nb);
-    bwd_layer(L_D1A, dT[T_YD1A], T[T_H1], T[T_YD1A], dT[T_H1], nb);
+    bwd_layer(L_D1B, dT[T_YD1B], T[T_YD1A], dT[T_YD1A], T[T_YD1A], nb);
+    bwd_layer(L_D1A, dT[T_YD1A], T[T_H1], dT[T_H1], nullptr, nb);
     up_bwd(T_H1, T_YD2B, nb);
-    bwd_layer(L_D2B, dT[T_YD2B], T[T_YD2A], T[T_YD2B], dT[T_YD2A], nb);
-    bwd_layer(L_D2A, dT[T_YD2A], T[T_H2], T[T_YD2A], dT[T_H2], nb);
+    bwd_layer(L_D2B, dT[T_YD2B], T[T_YD2A], dT[T_YD2A], T[T_YD2A], nb);
+    bwd_layer(L_D2A, dT[T_YD2A], T[T_H2], dT[T_H2], nullptr, nb);
     up_bwd(T_H2, T_Y3C, nb);
-    bwd_layer(L_B3C, dT[T_Y3C], T[T_Y3B], T[T_Y3C], dT[T_Y3B], nb);
-    bwd_layer(L_B3B, dT[T_Y3B], T[T_Y3A], T[T_Y3B], dT[T_Y3A], nb);
-    bwd_layer(L_B3A, dT[T_Y3A], T[T_P2], T[T_Y3A], dT[T_P2], nb);
+    bwd_layer(L_B3C, dT[T_Y3C], T[T_Y3B], dT[T_Y3B], T[T_Y3B], nb);
+    bwd_layer(L_B3B, dT[T_Y3B], T[T_Y3A], dT[T_Y3A], T[T_Y3A], nb);
+    bwd_layer(L_B3A, dT[T_Y3A], T[T_P2], dT[T_P2], nullptr, nb);
     pool_bwd_add(T_P2, T_H2, T_S2, nb);
-    bwd_layer(L_E2B, dT[T_S2], T[T_Y2A], T[T_S2], dT[T_Y2A], nb);
-    bwd_layer(L_E2A, dT[T_Y2A], T[T_P1], T[T_Y2A], dT[T_P1], nb);
+    bwd_layer(L_E2B, dT[T_S2], T[T_Y2A], dT[T_Y2A], T[T_Y2A], nb);
+    bwd_layer(L_E2A, dT[T_Y2A], T[T_P1], dT[T_P1], nullptr, nb);
     pool_bwd_add(T_P1, T_H1, T_S1, nb);
-    bwd_layer(L_E1B, dT[T_S1], T[T_Y1A], T[T_S1], dT[T_Y1A], nb);
-    bwd_layer(L_E1A, dT[T_Y1A], T[T_P0], T[T_Y1A], dT[T_P0], nb);
+    bwd_layer(L_E1B, dT[T_S1], T[T_Y1A], dT[T_Y1A], T[T_Y1A], nb);
+    bwd_layer(L_E1A, dT[T_Y1A], T[T_P0], dT[T_P0], nullptr, nb);
     pool_bwd_add(T_P0, T_H0, T_S0, nb);
-    bwd_layer(L_E0B, dT[T_S0], T[T_Y0A], T[T_S0], dT[T_Y0A], nb);
-    bwd_layer(L_E0A, dT[T_Y0A], T[T_X], T[T_Y0A], nullptr, nb);
+    bwd_layer(L_E0B, dT[T_S0], T[T_Y0A], dT[T_Y0A], T[T_Y0A], nb);
+    bwd_layer(L_E0A, dT[T_Y0A], T[T_X], nullptr, nullptr, nb);
+    UCK(cudaEventRecord(ev_dw, st_w));
+    UCK(cudaStreamWaitEvent(st, ev_dw, 0));
     check_err();
     double s = 0.0;
     for (int i = 0; i < 256; ++i) s += h_lpart[i];
@@ -1082,6 +1092,8 @@ int mm_unet_create(int grid, int batch, mm_unet** out) {
     u->G = grid;
     u->B = batch;
     UCK(cudaStreamCreateWithFlags(&u->st, cudaStreamNonBlocking));
+    UCK(cudaStreamCreateWithFlags(&u->st_w, cudaStreamNonBlocking));
+    for (cudaEvent_t* e : {&u->ev_dy, &u->ev_dw}) UCK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     for (int l = 0; l < 4; ++l) u->vol[l] = mmn::make_vol(grid >> l);
     size_t off = 0;
     for (int l = 0; l < MM_UNET_LAYERS; ++l) {
@@ -1135,7 +1147,10 @@ int mm_unet_create(int grid, int batch, mm_unet** out) {
     g_unet_error = u->err;
     for (void* q : u->allocs) cudaFree(q);
     if (u->h_lpart) cudaFreeHost(u->h_lpart);
-    if (u->st) cudaStreamDestroy(u->st);
+    for (cudaEvent_t e : {u->ev_dy, u->ev_dw})
+      if (e) cudaEventDestroy(e);
+    for (cudaStream_t q : {u->st, u->st_w})
+      if (q) cudaStreamDestroy(q);
     delete u;
     return rc;
   }
@@ -1145,13 +1160,16 @@ int mm_unet_create(int grid, int batch, mm_unet** out) {
 
 int mm_unet_destroy(mm_unet* u) {
   if (!u) return MM_ERR_ARG;
-  if (u->st) cudaStreamSynchronize(u->st);
+  for (cudaStream_t q : {u->st, u->st_w})
+    if (q) cudaStreamSynchronize(q);
   for (cudaGraphExec_t e : u->fwd_exec)
     if (e) cudaGraphExecDestroy(e);
   for (void* q : u->allocs) cudaFree(q);
   if (u->h_lpart) cudaFreeHost(u->h_lpart);
-  if (u->ev_after) cudaEventDestroy(u->ev_after);
-  if (u->st) cudaStreamDestroy(u->st);
+  for (cudaEvent_t e : {u->ev_after, u->ev_dy, u->ev_dw})
+    if (e) cudaEventDestroy(e);
+  for (cudaStream_t q : {u->st, u->st_w})
+    if (q) cudaStreamDestroy(q);
   delete u;
   return MM_OK;
 }
