@@ -49,15 +49,16 @@ def flatten(params: dict[str, np.ndarray]) -> np.ndarray:
     return np.ascontiguousarray(np.concatenate(parts))
 
 
-def unflatten(flat: np.ndarray) -> dict[str, np.ndarray]:
+def unflatten(flat: np.ndarray, copy: bool = True) -> dict[str, np.ndarray]:
+    """The layers' arrays of a flat vector; without `copy` they are parts of it."""
     out, k = {}, 0
     for name, _, ci, co, _ in LAYERS:
         n = 27 * ci * co
-        out[name + ".w"] = flat[k:k + n].reshape(27, ci, co).copy()
+        out[name + ".w"] = flat[k:k + n].reshape(27, ci, co)
         k += n
-        out[name + ".b"] = flat[k:k + co].copy()
+        out[name + ".b"] = flat[k:k + co]
         k += co
-    return out
+    return {name: a.copy() for name, a in out.items()} if copy else out
 
 
 def init_params(seed: int = 0) -> dict[str, np.ndarray]:
@@ -121,7 +122,7 @@ class UNet:
     def get_grads(self) -> dict[str, np.ndarray]:
         flat = np.empty(self.n_params, np.float32)
         self._check("mm_unet_get_grads", _abi.lib().mm_unet_get_grads(self.h, _f32p(flat)))
-        return unflatten(flat)
+        return unflatten(flat, copy=False)
 
     def forward(self, x: np.ndarray) -> np.ndarray:
         """x [nb, G, G, G, 4] -> prediction [nb, G, G, G] (output channel 0)."""
