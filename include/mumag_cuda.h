@@ -358,7 +358,8 @@ int mm_time_kernel(mm_problem* h, int kernel, int reps, double* ms_per_launch, d
  * (whose refinement steps are decided on the host). */
 #define MM_OPT_MIN_GRAPH 14
 /* MM_OPT_ENERGY_FF_LANES: lanes per magnetic row of the float-float energy kernel (1, 2, 4 or 8;
- * default 4; mm_autotune times each with L2 flushed and keeps the fastest). */
+ * default 1 from 64Ki magnetic rows on, 4 below; mm_autotune times each with L2 flushed and keeps the
+ * fastest). */
 #define MM_OPT_ENERGY_FF_LANES 15
 /* MM_OPT_COARSE_CYCLE (bit mask, default 0; mm_autotune keeps what is faster): with four levels, the
  * fused restriction at level 1 and the fused coarse correction, the V-cycle runs levels 1 .. 3 (the

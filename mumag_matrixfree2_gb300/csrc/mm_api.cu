@@ -255,7 +255,7 @@ struct mm_problem {
   bool eopsff_failed = false;      // an entry lies outside the range of the float-float pairs
   int energy_ff = -1;              // MM_OPT_ENERGY_FF
   mmk::NodesFF w_ff{};             // the node records it gathers
-  int eff_tpr = 4;                 // its lanes per magnetic row (mm_autotune)
+  int eff_tpr = 0;                 // its lanes per magnetic row (MM_OPT_ENERGY_FF_LANES, mm_autotune), 0: by size
   int min_fp32 = -1;               // MM_OPT_MIN_FP32
   double* d_Mn = nullptr;
   double* d_inv_M_rel = nullptr;
@@ -651,6 +651,10 @@ struct mm_problem {
     d.s.val = upload_as<T>(val);
     if (d.tpr == 1) d.stored = sptr[ns];
   }
+  // One lane a row reads the entries in whole lines and needs no merging of lanes, but small meshes have too few rows to
+  // hide the gathers: an evaluation with 1, 2 and 4 lanes takes 280, 322 and 351 us (1.03M magnetic rows), 79, 91 and 98
+  // (133k), but 62, 57 and 52 (9k).
+  int eff_lanes() const { return eff_tpr ? eff_tpr : eops.n_rows >= 65536 ? 1 : 4; }
   double red(int slot) {
     CK(cudaMemcpyAsync(&h_sc->red[slot], &d_sc->red[slot], sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -1589,7 +1593,7 @@ void enqueue_energy(mm_problem* h, const double* d_m, const double* d_U, const d
     mmk::k_split_ff<<<grid_elem(o.n_touched), BS, 0, h->st>>>(o.n_touched, o.touched, d_m, d_U, o.kx, o.ky, o.kz,
                                                                nf);
     LAUNCH_CHECK();
-    switch (h->eff_tpr) {
+    switch (h->eff_lanes()) {
       case 1: energy_ff_rows<1>(h, d_m, B, d_B, d_bias, d_g); break;
       case 2: energy_ff_rows<2>(h, d_m, B, d_B, d_bias, d_g); break;
       case 8: energy_ff_rows<8>(h, d_m, B, d_B, d_bias, d_g); break;
@@ -4152,7 +4156,7 @@ std::string tune_energy_ff(mm_problem* h, int reps) {
   CK(cudaEventCreate(&e1));
   std::string rep = "{\"us\":{";
   float best = 1e30f;
-  int best_tpr = h->eff_tpr;
+  int best_tpr = h->eff_lanes();
   for (int tpr : {1, 2, 4, 8}) {
     h->eff_tpr = tpr;
     enqueue_energy(h, h->d_m, h->d_U, B, nullptr, h->d_g);  // warm-up
@@ -4221,7 +4225,7 @@ int mm_get_option(mm_problem* h, int option, int* value) {
     case MM_OPT_COARSE_CYCLE: *value = h->coarse_cycle; return MM_OK;
     case MM_OPT_FUSE_RESTRICT: *value = h->fuse_restrict; return MM_OK;
     case MM_OPT_COARSE_FUSE: *value = h->coarse_fuse; return MM_OK;
-    case MM_OPT_ENERGY_FF_LANES: *value = h->eff_tpr; return MM_OK;
+    case MM_OPT_ENERGY_FF_LANES: *value = h->eff_lanes(); return MM_OK;
     case MM_OPT_MIN_GRAPH: *value = h->min_graph; return MM_OK;
     default: return MM_ERR_ARG;
   }
@@ -4352,7 +4356,7 @@ int mm_set_option(mm_problem* h, int option, int value) {
   }
   if (option == MM_OPT_ENERGY_FF_LANES) {
     if (value != 1 && value != 2 && value != 4 && value != 8) return MM_ERR_ARG;
-    if (h->eff_tpr != value) h->drop_min_graphs();
+    if (h->eff_lanes() != value) h->drop_min_graphs();
     h->eff_tpr = value;
     return MM_OK;
   }

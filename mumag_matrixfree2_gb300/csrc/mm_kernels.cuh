@@ -1511,7 +1511,23 @@ __device__ __forceinline__ void ff_madd(float ah, float al, float bh, float bl, 
   sl += err + e;
 }
 
+// (fl32(v), fl32(v - fl32(v))).  In integers where both parts are normal: three conversions and an add a value hold the
+// FP64 pipe for 64 clocks a warp, and were 41 of the 47 us in which 1.03M nodes' five values are split.  The
+// significand is rounded to its 24 upper bits (ties to even); what is left, at most 2^28 of its last places, is
+// converted with the same rounding and scaled exactly.
 __device__ __forceinline__ float2 ff_split(double v) {
+  const long long b = __double_as_longlong(v);
+  const int e = (int)(b >> 52) & 0x7ff;
+  if ((unsigned)(e - (1023 - 70)) <= 196u) {
+    const long long m = (b & 0xfffffffffffffLL) | (1LL << 52);
+    const int up = (int)(m >> 29), r = (int)(m & 0x1fffffff);
+    const int hi = up + (r + 0x0fffffff + (up & 1) >> 29);
+    const int lo = r - (hi - up << 29);
+    const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
+    const float h = __uint_as_float((unsigned)(e - 1023 + 127 - 1 << 23) + (unsigned)hi | sign);
+    const float l = (float)lo * __uint_as_float((unsigned)(e - 1023 - 52 + 127 << 23) | sign);
+    return make_float2(h, l);
+  }
   const float h = (float)v;
   return make_float2(h, (float)(v - (double)h));
 }
@@ -1550,9 +1566,12 @@ __device__ __forceinline__ void ff_shfl_add(float& sh, float& sl, int o) {
 }
 
 // g = (K m + G U + g_z) / V_mag on the magnetic rows; m.(g_quad + 2 g_z) -> red[R_E] (FP64).
-// TPR lanes per row (133k magnetic rows would give one thread per row too few warps to hide the
+// TPR lanes per row (a few thousand magnetic rows would give one thread per row too few warps to hide the
 // gather latency): lane q takes entries q, q + TPR, ..., and the row's float-float sums are merged
 // over its lanes by a fixed shuffle tree (FP32 shuffles and adds), so the result is deterministic.
+// What bounds it: the L1's wavefronts (three gathers and 44 bytes an entry) and, from memory, 44 bytes an entry.
+// 1.03M magnetic rows, with the splitting: 403 us an evaluation with four lanes and an FP64 end a row on one lane of
+// four, 351 with that end on whole warps, 280 with one lane.
 template <int TPR>
 __global__ void __launch_bounds__(BS) k_energy_grad_ff(EnergySellFF op, const float4* __restrict__ nh,
                                                        const float4* __restrict__ nl, const float2* __restrict__ nu,
@@ -1567,6 +1586,7 @@ __global__ void __launch_bounds__(BS) k_energy_grad_ff(EnergySellFF op, const fl
     Bz = Bd[2];
   }
   constexpr int RPB = BS / TPR;
+  __shared__ float2 s_row[TPR > 1 ? 3 * RPB : 1];
   const int q = threadIdx.x % TPR;
   double en = 0.0;
   for (int rb = blockIdx.x * RPB; rb < op.n_rows; rb += gridDim.x * RPB) {
@@ -1604,17 +1624,36 @@ __global__ void __launch_bounds__(BS) k_energy_grad_ff(EnergySellFF op, const fl
       ff_shfl_add(uyh, uyl, o);
       ff_shfl_add(uzh, uzl, o);
     }
-    if (valid && q == 0) {
-      // a - t k and then + u in float-float; one widening per component (the FP64 pipe issues a
-      // warp-wide instruction in 16 cycles whatever its active lanes)
+    if (q == 0) {  // a - t k and then + u in float-float
       ff_madd(-th, -tl, op.kfx.x, op.kfx.y, axh, axl);
       ff_madd(-th, -tl, op.kfy.x, op.kfy.y, ayh, ayl);
       ff_madd(-th, -tl, op.kfz.x, op.kfz.y, azh, azl);
       ff_add(axh, axl, uxh, uxl, axh, axl);
       ff_add(ayh, ayl, uyh, uyl, ayh, ayl);
       ff_add(azh, azl, uzh, uzl, azh, azl);
+    }
+    // From here on FP64, whose pipe a warp-wide instruction holds for 16 clocks whatever its active lanes: the rows'
+    // sums go through shared memory to the block's first warps, a lane a row.
+    if (TPR > 1) {
+      __syncthreads();  // the rows before have been read
+      if (q == 0) {
+        float2* const o = s_row + 3 * (threadIdx.x / TPR);
+        o[0] = make_float2(axh, axl);
+        o[1] = make_float2(ayh, ayl);
+        o[2] = make_float2(azh, azl);
+      }
+      __syncthreads();
+    }
+    const int rf = rb + threadIdx.x;
+    if (threadIdx.x < RPB && rf < op.n_rows) {
+      if (TPR > 1) {
+        const float2* const o = s_row + 3 * threadIdx.x;
+        axh = o[0].x, axl = o[0].y;
+        ayh = o[1].x, ayl = o[1].y;
+        azh = o[2].x, azl = o[2].y;
+      }
       const double ax = (double)axh + (double)axl, ay = (double)ayh + (double)ayl, az = (double)azh + (double)azl;
-      const int a = __ldg(op.rows + r);
+      const int a = __ldg(op.rows + rf);
       double bx = Bx, by = By, bz = Bz;
       if (Bbias) {
         bx += Bbias[3 * a];
