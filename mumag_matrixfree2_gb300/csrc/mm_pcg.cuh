@@ -606,8 +606,19 @@ __device__ __forceinline__ void pcoarse_a(const PcgArgs<TP, TV>& a, const PStep<
     for (int r = blockIdx.x; r < a.zr; r += gridDim.x) {
       const TV* zr = a.Z + (size_t)r * n;
       double acc = 0.0;
-#pragma unroll 4
-      for (int k = tb; k < n; k += BS) acc = fma((double)__ldg(zr + k), (double)b[k], acc);
+#pragma unroll 1
+      for (int k = tb; k < n; k += 8 * BS) {
+        TV m[8] = {}, v[8] = {};
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (k + j * BS < n) {
+            m[j] = __ldg(zr + k + j * BS);
+            v[j] = b[k + j * BS];
+          }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (k + j * BS < n) acc = fma((double)m[j], (double)v[j], acc);
+      }
       s_red[tb] = acc;
       asm volatile("barrier.sync 1, %0;" ::"n"(BS) : "memory");
       if (tb < 32) {
@@ -642,8 +653,19 @@ __device__ __forceinline__ void pdense(const PcgArgs<TP, TV>& a, const PStep<TV>
     TV acc = TV(0);
     if (row < st.A.n) {
       const TV* mr = a.M + (size_t)row * nc;
-#pragma unroll 4
-      for (int k = q; k < nc; k += 1 << lg) acc = fmaT<TV>(__ldg(mr + k), v[k], acc);
+#pragma unroll 1
+      for (int k = q; k < nc; k += 8 << lg) {
+        TV m[8] = {}, g[8] = {};
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (k + (j << lg) < nc) {
+            m[j] = __ldg(mr + k + (j << lg));
+            g[j] = v[k + (j << lg)];
+          }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (k + (j << lg) < nc) acc = fmaT<TV>(m[j], g[j], acc);
+      }
     }
 #pragma unroll 1
     for (int o = 1 << lg >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
