@@ -445,6 +445,7 @@ __device__ __forceinline__ void preduce(const PcgArgs<TP, TV>& a, int kind, PSca
       const int r0 = rb + 32 * (ug % WPB) + lane, r1 = r0 + BS;
       T ax[2] = {}, e0[2] = {}, e1[2] = {}, e2[2] = {}, e3[2] = {};
       float sl[2] = {};
+      TV e4[2] = {};
       // the rows' vector entries, in flight with the product's loads
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
@@ -463,6 +464,7 @@ __device__ __forceinline__ void preduce(const PcgArgs<TP, TV>& a, int kind, PSca
           e1[q] = (T)a.p[i];
           e2[q] = (T)a.Ap[i];
           e3[q] = (T)a.r[i];
+          if (a.xv) e4[q] = a.s0[i];
         } else if (INNER) {
           e0[q] = (T)a.xv[i];
           e1[q] = (T)a.s0[i];
@@ -510,7 +512,7 @@ __device__ __forceinline__ void preduce(const PcgArgs<TP, TV>& a, int kind, PSca
           acc.add(ri, ri);
           const TV rf = (TV)ri;
           if (MP) a.rv[i] = rf;
-          if (a.xv) a.xv[i] = a.s0[i] * rf;
+          if (a.xv) a.xv[i] = (kind == PS_STEP ? e4[q] : a.s0[i]) * rf;
         } else if (INNER) {
           const T yi = e0[q] + e1[q] * (e2[q] - ax[q]);
           a.z[i] = (TV)yi;
