@@ -1463,13 +1463,13 @@ void run_pcg_mp(mm_problem* h, double tol, int maxiter, int* iters, double* r2_o
   if (r2_out) *r2_out = h->h_sc->red[R_R2];
 }
 
-// b = D m on device (magnetic rows), b.b -> red[R_BB0]
-void enqueue_rhs(mm_problem* h, const double* m) {
+// b = D m on device (magnetic rows), b.b -> red[R_BB0] if asked for
+void enqueue_rhs(mm_problem* h, const double* m, bool norm = true) {
   const int N = h->N;
   if (!h->has_mask) CK(cudaMemsetAsync(h->d_b, 0, N * sizeof(double), h->st));
   mmk::k_rhs_s<<<grid_elem(h->eops.n_rows), BS, 0, h->st>>>(h->eops, m, h->d_b);
   LAUNCH_CHECK();
-  dot(h, N, h->d_b, nullptr, R_BB0);
+  if (norm) dot(h, N, h->d_b, nullptr, R_BB0);
 }
 
 void sub_mean(mm_problem* h, double* x) {
@@ -1521,14 +1521,25 @@ int run_mixed(mm_problem* h, double tol, int maxiter, int* iters, double* r2_out
 int solve_dev(mm_problem* h, const double* d_m, double* d_U, double tol, int maxiter, int* iters, double* rel_res,
               double* h_out = nullptr, cudaEvent_t x0_ready = nullptr) {
   if (!h->poisson_built) throw Fail{MM_ERR_STATE, "mm_build_poisson must be called before a solve"};
-  CK(cudaEventRecord(h->ev0, h->st));
-  enqueue_rhs(h, d_m);
-  if (x0_ready) CK(cudaStreamWaitEvent(h->st, x0_ready, 0));
-  if (d_U != h->d_x) CK(cudaMemcpyAsync(h->d_x, d_U, h->N * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
   const bool zero_mean = !h->has_mask;
+  const bool mixed = h->mixed && h->s32.built;
+  const bool mp = !mixed && h->fp32_precond && h->s32.built && multilevel(h, h->s32);
+  // The one-launch PCG takes the caller's U as its iterate and forms b.b itself: two copies and an inner product
+  // less in front of and behind it (10 us of a solve).
+  const bool direct = !mixed && !zero_mean && (mp ? persistent_ok(h, h->s32) && h->use_a0df() : persistent_ok(h, h->s64));
+  CK(cudaEventRecord(h->ev0, h->st));
+  enqueue_rhs(h, d_m, !direct);
+  if (x0_ready) CK(cudaStreamWaitEvent(h->st, x0_ready, 0));
+  struct Iterate {  // s64.x for this call
+    mm_problem* h;
+    Iterate(mm_problem* p, double* x) : h(p) { h->s64.x = x; }
+    ~Iterate() { h->s64.x = h->d_x; }
+  } iterate(h, direct ? d_U : h->d_x);
+  double* const x = h->s64.x;
+  if (d_U != x) CK(cudaMemcpyAsync(x, d_U, h->N * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
   if (zero_mean) {
     sub_mean(h, h->d_b);
-    sub_mean(h, h->d_x);
+    sub_mean(h, x);
   }
   int it = 0;
   double r2 = 0.0;
@@ -1536,19 +1547,19 @@ int solve_dev(mm_problem* h, const double* d_m, double* d_U, double tol, int max
   // the PCG paths queue their scalars copy and are read after the one wait below (it carries r.r,
   // the iteration count, tol2 and b.b)
   PcgPending pend;
-  if (h->mixed && h->s32.built) {
+  if (mixed) {
     run_mixed(h, tol, maxiter, &it, &r2);
     tol2_ref = tol * tol * h->red(R_BB);
-  } else if (h->fp32_precond && h->s32.built && multilevel(h, h->s32)) {
+  } else if (mp) {
     run_pcg_mp(h, tol, maxiter, nullptr, nullptr, &pend);
   } else {
     run_pcg<double>(h, h->s64, tol, maxiter, nullptr, nullptr, &pend);
   }
-  if (zero_mean) sub_mean(h, h->d_x);
-  if (d_U != h->d_x) CK(cudaMemcpyAsync(d_U, h->d_x, h->N * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
+  if (zero_mean) sub_mean(h, x);
+  if (d_U != x) CK(cudaMemcpyAsync(d_U, x, h->N * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
   CK(cudaEventRecord(h->ev1, h->st));
   if (h_out) {
-    CK(cudaMemcpyAsync(h_out, h->d_x, h->N * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+    CK(cudaMemcpyAsync(h_out, x, h->N * sizeof(double), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
   } else {
     CK(cudaEventSynchronize(h->ev1));
@@ -1561,7 +1572,7 @@ int solve_dev(mm_problem* h, const double* d_m, double* d_U, double tol, int max
   if (pend.S) {
     finish_pcg(h, pend, &it, &r2);
     tol2_ref = h->h_sc->tol2;
-    bb0 = h->h_sc->red[R_BB0];
+    bb0 = h->h_sc->red[direct ? R_BB : R_BB0];
   } else {
     bb0 = h->red(R_BB0);
   }
