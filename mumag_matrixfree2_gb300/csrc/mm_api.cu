@@ -1463,12 +1463,25 @@ void run_pcg_mp(mm_problem* h, double tol, int maxiter, int* iters, double* r2_o
   if (r2_out) *r2_out = h->h_sc->red[R_R2];
 }
 
+// Lanes a row of the FP64 right-hand side and energy below this many magnetic rows (one from there on): an energy
+// evaluation with 1, 2, 4 and 8 lanes takes 66, 54, 51 and 54 us (9k rows), 62, 56, 51 and 53 (3k); 102 and 114 with 1
+// and 2 lanes (133k).  The right-hand side of a solve with 1 and 4 lanes: 626 and 618 us a solve (9k rows).
+constexpr int OP_LANES = 4;
+constexpr int OP_LANES_ROWS = 65536;
+
+// b = D m on the magnetic rows; lanes a row as in enqueue_energy
+void rhs_rows(mm_problem* h, const double* m) {
+  const int n = h->eops.n_rows;
+  if (n < OP_LANES_ROWS) mmk::k_rhs_s<OP_LANES><<<grid_rows(n, OP_LANES), BS, 0, h->st>>>(h->eops, m, h->d_b);
+  else mmk::k_rhs_s<1><<<grid_elem(n), BS, 0, h->st>>>(h->eops, m, h->d_b);
+  LAUNCH_CHECK();
+}
+
 // b = D m on device (magnetic rows), b.b -> red[R_BB0] if asked for
 void enqueue_rhs(mm_problem* h, const double* m, bool norm = true) {
   const int N = h->N;
   if (!h->has_mask) CK(cudaMemsetAsync(h->d_b, 0, N * sizeof(double), h->st));
-  mmk::k_rhs_s<<<grid_elem(h->eops.n_rows), BS, 0, h->st>>>(h->eops, m, h->d_b);
-  LAUNCH_CHECK();
+  rhs_rows(h, m);
   if (norm) dot(h, N, h->d_b, nullptr, R_BB0);
 }
 
@@ -1613,9 +1626,13 @@ void enqueue_energy(mm_problem* h, const double* d_m, const double* d_U, const d
     LAUNCH_CHECK();
     return;
   }
-  mmk::k_energy_grad_s<<<grid_elem(h->eops.n_rows), BS, 0, h->st>>>(h->eops, d_m, d_U, h->d_Mn, B[0], B[1], B[2],
-                                                                     d_B, d_bias, h->inv_Vmag, d_g, h->d_sc,
-                                                                     h->d_part);
+  auto fp64 = [&](auto kern, int grid) {
+    kern<<<grid, BS, 0, h->st>>>(h->eops, d_m, d_U, h->d_Mn, B[0], B[1], B[2], d_B, d_bias, h->inv_Vmag, d_g, h->d_sc,
+                                 h->d_part);
+  };
+  const int n = h->eops.n_rows;
+  if (n < OP_LANES_ROWS) fp64(mmk::k_energy_grad_s<OP_LANES>, grid_rows(n, OP_LANES));
+  else fp64(mmk::k_energy_grad_s<1>, grid_elem(n));
   LAUNCH_CHECK();
 }
 
@@ -2079,8 +2096,7 @@ void enqueue_demag_nested(mm_problem* h, const double* m, double* U, double tol,
     mmk::k_zero_vec<<<grid_vec(N), BS, 0, h->st>>>(N, h->d_b);
     LAUNCH_CHECK();
   }
-  mmk::k_rhs_s<<<grid_elem(h->eops.n_rows), BS, 0, h->st>>>(h->eops, m, h->d_b);
-  LAUNCH_CHECK();
+  rhs_rows(h, m);
   dot(h, N, h->d_b, nullptr, R_BB0);
   if (!h->has_mask) {
     sub_mean(h, h->d_b);

@@ -1323,16 +1323,17 @@ struct EnergySell {
 
 // (exchange + anisotropy + magnetoelastic) v on row r: sum_k w v_j - q (k.v_j) k (+ mex v_j,x, mey v_j,y);
 // with a single easy axis the anisotropy sum is accumulated as a scalar and applied once
-__device__ __forceinline__ void exch_aniso_sell(const EnergySell& op, int r, const double* __restrict__ v,
-                                                double& ax, double& ay, double& az) {
+// (t; exch_aniso_end).  Here a lane's share of the row, the entries q, q + TPR, ...
+template <int TPR>
+__device__ __forceinline__ void exch_aniso_lane(const EnergySell& op, int r, int q, const double* __restrict__ v,
+                                                double& ax, double& ay, double& az, double& t) {
   const int s = r >> 5, l = r & 31;
   const int base = __ldg(op.sptr + s), wd = (__ldg(op.sptr + s + 1) - base) >> 5;
-  ax = ay = az = 0.0;
+  ax = ay = az = t = 0.0;
   if (op.single_axis) {
     const double kx = op.kax[3 * op.axis0], ky = op.kax[3 * op.axis0 + 1], kz = op.kax[3 * op.axis0 + 2];
-    double t = 0.0;
 #pragma unroll 3
-    for (int k = 0; k < wd; ++k) {
+    for (int k = q; k < wd; k += TPR) {
       const int at = base + (k << 5) + l;
       const int j = __ldg(op.col + at);
       const double vx = __ldg(v + 3 * j), vy = __ldg(v + 3 * j + 1), vz = __ldg(v + 3 * j + 2);
@@ -1346,22 +1347,19 @@ __device__ __forceinline__ void exch_aniso_sell(const EnergySell& op, int r, con
         ay = fma(__ldg(op.mey + at), vy, ay);
       }
     }
-    ax = fma(-t, kx, ax);
-    ay = fma(-t, ky, ay);
-    az = fma(-t, kz, az);
   } else {
 #pragma unroll 2
-    for (int k = 0; k < wd; ++k) {
+    for (int k = q; k < wd; k += TPR) {
       const int at = base + (k << 5) + l;
       const int j = __ldg(op.col + at);
       const int g = __ldg(op.mat + at);
       const double kx = op.kax[3 * g], ky = op.kax[3 * g + 1], kz = op.kax[3 * g + 2];
       const double vx = __ldg(v + 3 * j), vy = __ldg(v + 3 * j + 1), vz = __ldg(v + 3 * j + 2);
       const double wk = __ldg(op.w + at);
-      const double t = -__ldg(op.q + at) * fma(kz, vz, fma(ky, vy, kx * vx));
-      ax = fma(t, kx, fma(wk, vx, ax));
-      ay = fma(t, ky, fma(wk, vy, ay));
-      az = fma(t, kz, fma(wk, vz, az));
+      const double tk = -__ldg(op.q + at) * fma(kz, vz, fma(ky, vy, kx * vx));
+      ax = fma(tk, kx, fma(wk, vx, ax));
+      ay = fma(tk, ky, fma(wk, vy, ay));
+      az = fma(tk, kz, fma(wk, vz, az));
       if (op.mex) {
         ax = fma(__ldg(op.mex + at), vx, ax);
         ay = fma(__ldg(op.mey + at), vy, ay);
@@ -1370,7 +1368,31 @@ __device__ __forceinline__ void exch_aniso_sell(const EnergySell& op, int r, con
   }
 }
 
+__device__ __forceinline__ void exch_aniso_end(const EnergySell& op, double t, double& ax, double& ay, double& az) {
+  if (!op.single_axis) return;
+  ax = fma(-t, op.kax[3 * op.axis0], ax);
+  ay = fma(-t, op.kax[3 * op.axis0 + 1], ay);
+  az = fma(-t, op.kax[3 * op.axis0 + 2], az);
+}
+
+__device__ __forceinline__ void exch_aniso_sell(const EnergySell& op, int r, const double* __restrict__ v,
+                                                double& ax, double& ay, double& az) {
+  double t;
+  exch_aniso_lane<1>(op, r, 0, v, ax, ay, az, t);
+  exch_aniso_end(op, t, ax, ay, az);
+}
+
+template <int TPR>
+__device__ __forceinline__ double lanes_sum(double v) {
+#pragma unroll
+  for (int o = TPR / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// The FP64 operators take TPR lanes a row (rows by one thread: a chain of dependent loads and FP64 operations that
+// a small mesh has too few warps to hide; by several: 16 clocks of the FP64 pipe for every step of a reduction).
 // g = (K m + G U + g_z) / V_mag on the magnetic rows; m.(g_quad + 2 g_z) -> red[R_E]
+template <int TPR>
 __global__ void __launch_bounds__(BS) k_energy_grad_s(EnergySell op, const double* __restrict__ m,
                                                       const double* __restrict__ U, const double* __restrict__ Mn,
                                                       double Bx, double By, double Bz, const double* __restrict__ Bd,
@@ -1382,20 +1404,35 @@ __global__ void __launch_bounds__(BS) k_energy_grad_s(EnergySell op, const doubl
     Bz = Bd[2];
   }
   double en = 0.0;
-  for (int r = blockIdx.x * BS + threadIdx.x; r < op.n_rows; r += gridDim.x * BS) {
-    double ax, ay, az;
-    exch_aniso_sell(op, r, m, ax, ay, az);
-    const int s = r >> 5, l = r & 31;
-    const int base = __ldg(op.sptr + s), wd = (__ldg(op.sptr + s + 1) - base) >> 5;
-    double ux = 0, uy = 0, uz = 0;
+  constexpr int RPB = BS / TPR;
+  const int q = threadIdx.x % TPR;
+  for (int rb = blockIdx.x * RPB; rb < op.n_rows; rb += gridDim.x * RPB) {
+    const int r = rb + threadIdx.x / TPR;
+    const bool valid = r < op.n_rows;
+    if (TPR == 1 && !valid) break;
+    double ax = 0, ay = 0, az = 0, t = 0, ux = 0, uy = 0, uz = 0;
+    if (valid) {
+      exch_aniso_lane<TPR>(op, r, q, m, ax, ay, az, t);
+      const int s = r >> 5, l = r & 31;
+      const int base = __ldg(op.sptr + s), wd = (__ldg(op.sptr + s + 1) - base) >> 5;
 #pragma unroll 3
-    for (int k = 0; k < wd; ++k) {
-      const int at = base + (k << 5) + l;
-      const double u = __ldg(U + __ldg(op.col + at));
-      ux = fma(__ldg(op.gx + at), u, ux);
-      uy = fma(__ldg(op.gy + at), u, uy);
-      uz = fma(__ldg(op.gz + at), u, uz);
+      for (int k = q; k < wd; k += TPR) {
+        const int at = base + (k << 5) + l;
+        const double u = __ldg(U + __ldg(op.col + at));
+        ux = fma(__ldg(op.gx + at), u, ux);
+        uy = fma(__ldg(op.gy + at), u, uy);
+        uz = fma(__ldg(op.gz + at), u, uz);
+      }
     }
+    if (TPR > 1) {  // one sum a component
+      ax = lanes_sum<TPR>(ax + ux);
+      ay = lanes_sum<TPR>(ay + uy);
+      az = lanes_sum<TPR>(az + uz);
+      t = lanes_sum<TPR>(t);
+      ux = uy = uz = 0.0;
+      if (!valid || q) continue;
+    }
+    exch_aniso_end(op, t, ax, ay, az);
     const int a = __ldg(op.rows + r);
     double bx = Bx, by = By, bz = Bz;
     if (Bbias) {
@@ -1454,19 +1491,27 @@ __global__ void __launch_bounds__(BS) k_apply_P_s(EnergySell op, const double* _
 }
 
 // b = D m on the magnetic rows (other rows untouched)
+template <int TPR>
 __global__ void __launch_bounds__(BS) k_rhs_s(EnergySell op, const double* __restrict__ m, double* __restrict__ b) {
-  for (int r = blockIdx.x * BS + threadIdx.x; r < op.n_rows; r += gridDim.x * BS) {
-    const int s = r >> 5, l = r & 31;
-    const int base = __ldg(op.sptr + s), wd = (__ldg(op.sptr + s + 1) - base) >> 5;
+  constexpr int RPB = BS / TPR;
+  const int q = threadIdx.x % TPR;
+  for (int rb = blockIdx.x * RPB; rb < op.n_rows; rb += gridDim.x * RPB) {
+    const int r = rb + threadIdx.x / TPR;
+    const bool valid = r < op.n_rows;
     double acc = 0.0;
+    if (valid) {
+      const int s = r >> 5, l = r & 31;
+      const int base = __ldg(op.sptr + s), wd = (__ldg(op.sptr + s + 1) - base) >> 5;
 #pragma unroll 3
-    for (int k = 0; k < wd; ++k) {
-      const int at = base + (k << 5) + l;
-      const int j = __ldg(op.col + at);
-      acc += __ldg(op.dx + at) * __ldg(m + 3 * j) + __ldg(op.dy + at) * __ldg(m + 3 * j + 1) +
-             __ldg(op.dz + at) * __ldg(m + 3 * j + 2);
+      for (int k = q; k < wd; k += TPR) {
+        const int at = base + (k << 5) + l;
+        const int j = __ldg(op.col + at);
+        acc += __ldg(op.dx + at) * __ldg(m + 3 * j) + __ldg(op.dy + at) * __ldg(m + 3 * j + 1) +
+               __ldg(op.dz + at) * __ldg(m + 3 * j + 2);
+      }
     }
-    b[__ldg(op.rows + r)] = acc;
+    acc = lanes_sum<TPR>(acc);
+    if (valid && q == 0) b[__ldg(op.rows + r)] = acc;
   }
 }
 
