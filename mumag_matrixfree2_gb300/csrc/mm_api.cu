@@ -1149,15 +1149,13 @@ bool persistent_ok(mm_problem* h, const SolverT<T>& F) {
          one_launch_rows<T>(h->N);
 }
 
-// Blocks: one per 256 rows (FP64 V-cycle: two FP64 operations a clock an SM) or 512 (FP32: the 45,570-node
-// particle takes 628 us with one per 512, 713 with one per 1024, and leaves SMs to other streams' problems),
-// at most one per SM.  Up to 16 as one cluster of 16, whose hardware barrier costs a quarter of the grid's.
+// Blocks: one per 256 rows, at most one per SM (a solve with one per 128, 256, 384 and 512 rows: 59,319 nodes 617,
+// 615, 616 and 664 us, FP32 V-cycle 553, 553, 552 and 583; 45,570 nodes 541, 540, 563 and 602, FP32 482, 483, 483 and
+// 492).  Up to 16 as one cluster of 16, whose hardware barrier costs a quarter of the grid's.
 constexpr int PCG_CLUSTER = 16;
 
-template <class TV>
 int persistent_blocks(mm_problem* h) {
-  const int rows = sizeof(TV) == 8 ? 256 : 512;
-  const int want = std::min((h->N + rows - 1) / rows, h->pcg_cap);
+  const int want = std::min((h->N + 255) / 256, h->pcg_cap);
   return std::max(want, PCG_CLUSTER);
 }
 
@@ -1184,7 +1182,7 @@ int persistent_args(mm_problem* h, SolverT<TP>& S, SolverT<TV>& F, mmk::PcgArgs<
   const int bit = sizeof(TV) == 8 ? 0 : 1;
   const bool use_rf = (h->fuse_restrict >> bit) & 1;
   const bool fused = F.fused && ((h->coarse_fuse >> bit) & 1);
-  const int blocks = persistent_blocks<TV>(h);
+  const int blocks = persistent_blocks(h);
   a.cluster = blocks <= PCG_CLUSTER;
   a.n = h->N;
   a.G = grid_ilp(h->N);
