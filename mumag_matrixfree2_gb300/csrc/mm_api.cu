@@ -575,7 +575,6 @@ struct mm_problem {
       d.c.val = upload_as<T>(A.val);
       d.stored = A.nnz();
       d.s.n = A.n_rows;
-      upload_lanes<T>(A, d);
       return d;
     }
     upload_sell<T>(A, d);
@@ -601,19 +600,25 @@ struct mm_problem {
       sptr[s + 1] = sptr[s] + 64 * ((w + 1) / 2);  // paired entries (mmk::SellT)
     }
     std::vector<int> col(sptr[ns], 0);
-    std::vector<double> val(sptr[ns], 0.0);
-    for (int r = 0; r < A.n_rows; ++r) {
-      const int s = r / per, w2 = (sptr[s + 1] - sptr[s]) / 32, len = A.ptr[r + 1] - A.ptr[r];
-      for (int k = 0; k < t * w2; ++k) {
-        const size_t at = (size_t)sptr[s] + 64 * (k / t / 2) + 2 * (r % per * t + k % t) + k / t % 2;
-        if (len > 0) col[at] = A.col[A.ptr[r] + std::min(k, len - 1)];  // padding: value 0, a column of the row
-        if (k < len) val[at] = A.val[A.ptr[r] + k];
+    std::vector<T> val(sptr[ns], T(0));
+    mm::parallel_rows(A.n_rows, sptr[ns], [&](int64_t r0, int64_t r1) {
+      for (int r = (int)r0; r < (int)r1; ++r) {
+        const int s = r / per, w2 = (sptr[s + 1] - sptr[s]) / 32, len = A.ptr[r + 1] - A.ptr[r];
+        if (len == 0) continue;
+        const int* const c = &A.col[A.ptr[r]];
+        const double* const v = &A.val[A.ptr[r]];
+        for (int q = 0; q < t; ++q)
+          for (int i = 0, k = q; i < w2; ++i, k += t) {
+            const size_t at = (size_t)sptr[s] + 64 * (i / 2) + 2 * (r % per * t + q) + i % 2;
+            col[at] = c[std::min(k, len - 1)];  // padding: value 0, a column of the row
+            if (k < len) val[at] = (T)v[k];
+          }
       }
-    }
+    });
     o.n = A.n_rows;
     o.sptr = upload(sptr);
     o.col = upload(col);
-    o.val = upload_as<T>(val);
+    o.val = upload(val);
   }
   // sliced ELL (mmk::SellT): slices of 32 rows, entries paired, padding with value 0 and a valid column
   template <class T>
@@ -808,6 +813,49 @@ bool folded(const mm_problem* h, const SolverT<T>& S, int l) {
   return ((h->fuse_restrict >> bit) & 1) && S.lv[l].G.nnz > 0 && S.lv[l].Rf.nnz > 0 &&
          l < (S.fused && ((h->coarse_fuse >> bit) & 1) ? L - 2 : L - 1) &&
          (l > 0 || (int64_t)grid_ilp(h->N) * mmk::CHUNK >= h->N);  // pfold0 makes one round of the grid's blocks
+}
+
+// f(operator, host copy, name) for the operators of level l below the coarsest that a V-cycle reads (level 0's A,
+// always sliced ELL, left out), and f_not for those it does not
+template <class T, class F, class N>
+void level_operators(mm_problem* h, SolverT<T>& S, int l, F&& f, N&& f_not) {
+  const int L = (int)S.lv.size(), bit = sizeof(T) == 8 ? 0 : 1;
+  auto& c = S.lv[l];
+  const bool on = l < (S.fused && ((h->coarse_fuse >> bit) & 1) ? L - 2 : L - 1);
+  const bool rf = ((h->fuse_restrict >> bit) & 1) && c.Rf.nnz > 0, g = folded(h, S, l);
+  auto go = [&](bool used, DevMatT<T>& M, const mm::HostCSR& host, const char* name) {
+    if (used) f(M, host, name);
+    else f_not(M, host, name);
+  };
+  if (l > 0) go(on && !(rf && g), c.A, h->amg_h[l].A, "A");
+  if (l == L - 1) return;
+  go(on && !rf, c.R, h->amg_h[l].R, "R");
+  go(on && !g, c.P, h->amg_h[l].P, "P");
+  if (c.Rf.nnz > 0 && (int)h->rf_host.size() > l) go(on && rf, c.Rf, h->rf_host[l], "Rf");
+  if (c.G.nnz > 0) go(on && g, c.G, h->g_host[l], "G");
+}
+
+// The layouts that the one-launch PCG reads, for the operators that it would read now; called wherever that changes
+// (never inside a capture).
+template <class T>
+void ensure_lanes(mm_problem* h, SolverT<T>& S) {
+  const bool inner = std::is_same<T, float>::value;
+  if (!S.built || inner != (h->mixed || h->fp32_precond)) return;
+  for (int l = 0; l < (int)S.lv.size() - 1; ++l)
+    level_operators(h, S, l, [&](DevMatT<T>& M, const mm::HostCSR& host, const char*) { h->upload_lanes<T>(host, M); },
+                    [](DevMatT<T>&, const mm::HostCSR&, const char*) {});
+}
+
+template <class T>
+bool lanes_ready(mm_problem* h, SolverT<T>& S) {
+  bool ok = true;
+  for (int l = 0; l < (int)S.lv.size() - 1; ++l)
+    level_operators(h, S, l, [&](DevMatT<T>& M, const mm::HostCSR&, const char*) {
+      int lg = 0;
+      while ((1 << lg) < M.tpr) ++lg;
+      ok = ok && (lg == 0 ? M.s.sptr : M.lanes[lg - 1].sptr) != nullptr;
+    }, [](DevMatT<T>&, const mm::HostCSR&, const char*) {});
+  return ok;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1144,9 +1192,9 @@ mmk::POp<T> persistent_op(const DevMatT<T>& M) {
 }
 
 template <class T>
-bool persistent_ok(mm_problem* h, const SolverT<T>& F) {
+bool persistent_ok(mm_problem* h, SolverT<T>& F) {
   return h->use_graph && !h->prof && h->pcg_cap > 0 && multilevel(h, F) && (int)F.lv.size() <= mmk::PLEV &&
-         one_launch_rows<T>(h->N);
+         one_launch_rows<T>(h->N) && lanes_ready(h, F);
 }
 
 // Blocks: one per 256 rows, at most one per SM (a solve with one per 128, 256, 384 and 512 rows: 59,319 nodes 617,
@@ -3134,6 +3182,15 @@ bool fold_rows(int l, int64_t n) {
   return n <= (l == 0 ? 131072 : sizeof(T) == 8 ? 262144 : 65536);
 }
 
+// fused coarse correction only where the dense factors stay small: Z = Ainv M costs nc^2 n host FLOPs, W and Z hold
+// n nc each
+bool coarse_factors(const mm_problem* h) {
+  const int L = (int)h->amg_h.size();
+  if (L < 3) return false;
+  const double n = h->amg_h[L - 2].A.n_rows, nc = h->amg_h[L - 1].A.n_rows;
+  return nc <= 256 && n * nc <= 4194304.0;
+}
+
 // Upload the hierarchy in precision T and allocate the solver's vectors.
 template <class T>
 void build_solver(mm_problem* h, SolverT<T>& S, const mm::HostCSR& A, bool amg, int precond_type) {
@@ -3180,9 +3237,12 @@ void build_solver(mm_problem* h, SolverT<T>& S, const mm::HostCSR& A, bool amg, 
       h->rf_prec = precond_type;
       for (mm::AmgLevel& hl : h->amg_h) hl.RA = mm::HostCSR{};  // its one use is above
     }
+    const int fold_to = coarse_factors(h) ? L - 2 : L - 1;  // the factors replace the two coarsest levels
     for (int l = 0; l < L - 1; ++l) {
       S.lv[l].Rf = h->upload_mat<T>(h->rf_host[l]);
+      if (l >= fold_to) continue;
       if (!fold_rows<T>(l, h->amg_h[l].A.n_rows)) continue;
+      if (sizeof(T) == 8 && (h->mixed || h->fp32_precond)) continue;  // its V-cycle takes no part in the solves
       const mm::AmgLevel& hl = h->amg_h[l];
       mm::HostCSR& g = h->g_host[l];
       if (g.n_rows == 0) {
@@ -3212,11 +3272,7 @@ void build_solver(mm_problem* h, SolverT<T>& S, const mm::HostCSR& A, bool amg, 
   S.z = h->alloc<T>(h->N);
   S.p = h->alloc<T>(h->N);
   S.Ap = h->alloc<T>(h->N);
-  if (amg && L >= 3) {
-    // only where the dense factors stay small: Z = Ainv M costs nc^2 n host FLOPs, W and Z hold n nc each
-    const double n = h->amg_h[L - 2].A.n_rows, nc = h->amg_h[L - 1].A.n_rows;
-    if (nc <= 256 && n * nc <= 4194304.0) build_fused_coarse<T>(h, S, precond_type);
-  }
+  if (amg && coarse_factors(h)) build_fused_coarse<T>(h, S, precond_type);
   if (amg && L == 4 && S.fused) {
     // the one-launch coarse cycle: a grid that is co-resident (the cooperative launch checks it) and
     // the barrier it synchronises on
@@ -3231,6 +3287,7 @@ void build_solver(mm_problem* h, SolverT<T>& S, const mm::HostCSR& A, bool amg, 
     }
   }
   S.built = true;
+  ensure_lanes(h, S);
 }
 
 // =============================================================================================
@@ -4028,6 +4085,7 @@ float time_ms(mm_problem* h, int reps, const std::function<void()>& f) {
 // side and no tolerance; per V-cycle), else V-cycles back to back.
 template <class T>
 float vcycle_ms(mm_problem* h, SolverT<T>& S, int reps) {
+  ensure_lanes(h, S);
   const bool mp = h->fp32_precond && std::is_same<T, float>::value;
   const bool solves = std::is_same<T, float>::value ? (h->mixed || mp) : !(h->mixed || h->fp32_precond);
   if (!solves || !persistent_ok(h, S) || (mp && !h->use_a0df()))
@@ -4092,17 +4150,9 @@ void tune_solver(mm_problem* h, SolverT<T>& S, int reps, std::string& rep) {
   if (!S.built || !multilevel(h, S)) return;
   const int L = (int)S.lv.size();
   for (int l = 0; l < L; ++l) {
-    auto& c = S.lv[l];
-    const int bit = sizeof(T) == 8 ? 0 : 1;
-    const bool rf = ((h->fuse_restrict >> bit) & 1) && c.Rf.nnz > 0;
-    const bool on = l < (S.fused && ((h->coarse_fuse >> bit) & 1) ? L - 2 : L - 1), g = folded(h, S, l);
-    if (l > 0) tune_csr<T>(h, S, c.A, h->amg_h[l].A, reps, "A", l, on && !(rf && g), rep);
-    if (l < L - 1) {
-      tune_csr<T>(h, S, c.R, h->amg_h[l].R, reps, "R", l, on && !rf, rep);
-      tune_csr<T>(h, S, c.P, h->amg_h[l].P, reps, "P", l, on && !g, rep);
-      if (c.Rf.nnz > 0 && (int)h->rf_host.size() > l) tune_csr<T>(h, S, c.Rf, h->rf_host[l], reps, "Rf", l, on && rf, rep);
-      if (c.G.nnz > 0) tune_csr<T>(h, S, c.G, h->g_host[l], reps, "G", l, on && g, rep);
-    }
+    level_operators(h, S, l, [&](DevMatT<T>& M, const mm::HostCSR& host, const char* tag) {
+      tune_csr<T>(h, S, M, host, reps, tag, l, true, rep);
+    }, [&](DevMatT<T>& M, const mm::HostCSR& host, const char* tag) { tune_csr<T>(h, S, M, host, reps, tag, l, false, rep); });
   }
   drop_graph(S);
 }
@@ -4256,6 +4306,15 @@ int mm_get_option(mm_problem* h, int option, int* value) {
   }
 }
 
+// after an option that changes the operators that a V-cycle reads
+static int relayout(mm_problem* h) {
+  return guarded(h, [&] {
+    ensure_lanes(h, h->s64);
+    ensure_lanes(h, h->s32);
+    return MM_OK;
+  });
+}
+
 int mm_set_option(mm_problem* h, int option, int value) {
   if (!h) return MM_ERR_ARG;
   if (option == MM_OPT_GRAPH) {
@@ -4308,7 +4367,7 @@ int mm_set_option(mm_problem* h, int option, int value) {
       drop_graph(h->s32);
     }
     h->coarse_fuse = value;
-    return MM_OK;
+    return relayout(h);
   }
   if (option == MM_OPT_ENERGY_FF) {
     if (value < -1 || value > 1) return MM_ERR_ARG;
@@ -4322,7 +4381,7 @@ int mm_set_option(mm_problem* h, int option, int value) {
       drop_graph(h->s32);
     }
     h->fuse_restrict = value;
-    return MM_OK;
+    return relayout(h);
   }
   if (option == MM_OPT_SA_FACTOR_E3) {
     if (value < 0 || value > 1000) return MM_ERR_ARG;
@@ -4350,18 +4409,10 @@ int mm_set_option(mm_problem* h, int option, int value) {
         const int L = (int)S.lv.size();
         for (int l = 0; l < L; ++l) {
           auto& c = S.lv[l];
-          auto set = [&](auto& M, const mm::HostCSR& host) {
-            if (M.c.n == 0 || M.tpr == 1) return;
-            M.tpr = value;
-            h->upload_lanes(host, M);
-          };
-          set(c.A, h->amg_h[l].A);
-          if (l == L - 1) continue;
-          set(c.R, h->amg_h[l].R);
-          set(c.P, h->amg_h[l].P);
-          if (c.Rf.nnz > 0) set(c.Rf, h->rf_host[l]);
-          if (c.G.nnz > 0) set(c.G, h->g_host[l]);
+          for (auto* M : {&c.A, &c.R, &c.P, &c.Rf, &c.G})
+            if (M->c.n > 0 && M->tpr != 1) M->tpr = value;
         }
+        ensure_lanes(h, S);
         drop_graph(S);
       };
       set_all(h->s64);

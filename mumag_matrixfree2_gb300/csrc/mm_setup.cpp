@@ -43,6 +43,11 @@ static void parallel_chunks(int64_t n, int nt, F&& f) {
   for (auto& x : th) x.join();
 }
 
+void parallel_rows(int64_t n, int64_t work, const std::function<void(int64_t, int64_t)>& f) {
+  parallel_chunks(n, (int)std::min<int64_t>(setup_threads(work), std::max<int64_t>(n, 1)),
+                  [&](int, int64_t a, int64_t b) { f(a, b); });
+}
+
 // out = the concatenation of parts (in order), each part copied by its own thread
 template <class V, class P>
 static void concat_parallel(const std::vector<P>& parts, V& out) {

@@ -2,6 +2,7 @@
 // order, assembly of the compressed-row operators and the smoothed-aggregation hierarchy.
 #pragma once
 
+#include <functional>
 #include <cstdint>
 #include <memory>
 #include <new>
@@ -133,6 +134,8 @@ HostCSR fused_restriction_ra(const HostCSR& R, const HostCSR& RA, const std::vec
 // G = [2S - S A S | (I - S A) P], S = diag(s): from a level's right-hand side and the coarse correction, stacked with
 // the latter from row `offset` on, to the post-smoothed iterate
 HostCSR folded_prolongation(const HostCSR& A, const HostCSR& P, const std::vector<double>& s, int offset);
+// f(begin, end) on chunks of [0, n) by the setup's host threads (`work`: its items, for their number)
+void parallel_rows(int64_t n, int64_t work, const std::function<void(int64_t, int64_t)>& f);
 std::vector<double> dense_inverse(const HostCSR& A);  // row-major n x n; throws on singular
 
 }  // namespace mm
