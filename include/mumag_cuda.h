@@ -339,7 +339,8 @@ int mm_time_kernel(mm_problem* h, int kernel, int reps, double* ms_per_launch, d
 /* MM_OPT_FUSE_RESTRICT (bit mask, default 3): the V-cycle restricts with R_l (I - A_l S_l), formed
  * once on the host, instead of a residual pass A_l followed by R_l: the pre-smoothing from zero
  * makes x_l = S_l b_l, so b_{l+1} = R_l (b_l - A_l x_l) is one product with one operator (one kernel
- * less per level, and fewer bytes than A_l and R_l together).  Bit 0 the FP64 solver, bit 1 the FP32
+ * less per level, and fewer bytes than A_l and R_l together).  Small levels then also take prolongation
+ * and post-smoothing as one product.  Bit 0 the FP64 solver, bit 1 the FP32
  * one; mm_autotune keeps a bit only if the V-cycle is faster with it. */
 #define MM_OPT_FUSE_RESTRICT 12
 /* MM_OPT_ENERGY_FF: energy and gradient evaluations in float-float (every stored value and the vectors

@@ -136,9 +136,9 @@ struct SolverT {
   int sms = 0;
 };
 
-// Sizes whose PCG runs as one launch (V-cycle in T).  FP64: all measured (1,331 to 1,601,613 rows: 316 against
-// 469 us, 6.24 against 6.69 ms a solve).  FP32: up to 3/4 Mi rows (357,911 rows 1.68 against 1.78 ms; 1,601,613
-// rows 5.17 against 4.96 ms: streaming FP32 operators wants the 2048 threads an SM of the separate kernels).
+// Sizes whose PCG runs as one launch (V-cycle in T).  FP64: all measured (1,331 to 1,601,613 rows: 239 us a solve
+// against 469 as separate kernels, 5.83 against 6.69 ms).  FP32: up to 3/4 Mi rows (357,911 rows 1.55 against 1.78 ms;
+// 1,601,613 rows 5.17 against 4.96 ms: streaming FP32 operators wants the 2048 threads an SM of the separate kernels).
 template <class T>
 bool one_launch_rows(int64_t n) {
   return sizeof(T) == 8 || n <= 786432;
@@ -1210,7 +1210,8 @@ int persistent_blocks(mm_problem* h) {
 // One solve or minimization in flight.  Their number on the device decides how each runs its PCG, so that
 // several threads' problems share the GPU: alone on every SM, with one or two others on a third of them each,
 // and with more as separate kernels, whose many small launches overlap (48 particles on 16 threads, FP32
-// V-cycle: 16.3 s with every SM for each, 13.2 s with a cluster of 16 blocks each, 11.1 s as separate kernels).
+// V-cycle: 16.3 s with every SM for each, 13.2 s with a cluster of 16 blocks each, 11.1 s as separate kernels, now
+// 10.2).
 // The results are the same bits.
 std::atomic<int> g_solving[64];
 
