@@ -1191,12 +1191,6 @@ mmk::POp<T> persistent_op(const DevMatT<T>& M) {
   return o;
 }
 
-template <class T>
-bool persistent_ok(mm_problem* h, SolverT<T>& F) {
-  return h->use_graph && !h->prof && h->pcg_cap > 0 && multilevel(h, F) && (int)F.lv.size() <= mmk::PLEV &&
-         one_launch_rows<T>(h->N) && lanes_ready(h, F);
-}
-
 // Blocks: one per 256 rows, at most one per SM (a solve with one per 128, 256, 384 and 512 rows: 59,319 nodes 617,
 // 615, 616 and 664 us, FP32 V-cycle 553, 553, 552 and 583; 45,570 nodes 541, 540, 563 and 602, FP32 482, 483, 483 and
 // 492).  Up to 16 as one cluster of 16, whose hardware barrier costs a quarter of the grid's.
@@ -1205,6 +1199,25 @@ constexpr int PCG_CLUSTER = 16;
 int persistent_blocks(mm_problem* h) {
   const int want = std::min((h->N + 255) / 256, h->pcg_cap);
   return std::max(want, PCG_CLUSTER);
+}
+
+// Dynamic shared memory of a block: its share of the partials of eight warps and of b.b's, 2 KB each, which it folds, and
+// with level 0 folded its rows of z.  The largest: 4096 partials (2.1M rows and more) over a third of the SMs, 164 KB.
+constexpr size_t PCG_SMEM = 200 * 1024;
+
+template <class T>
+size_t persistent_smem(mm_problem* h, const SolverT<T>& F) {
+  const int blocks = persistent_blocks(h), G = grid_ilp(h->N), kshift = red_kshift(h->N);
+  const int parts = (G * mmk::WPB) >> kshift, dots = std::min(G, g_vec_cap);
+  size_t bytes = (size_t)((std::max(kshift ? parts : 0, dots) + blocks - 1) / blocks) * BS * sizeof(double);
+  if (folded(h, F, 0)) bytes += (size_t)((parts + blocks - 1) / blocks << kshift) * 64 * sizeof(T);
+  return bytes;
+}
+
+template <class T>
+bool persistent_ok(mm_problem* h, SolverT<T>& F) {
+  return h->use_graph && !h->prof && h->pcg_cap > 0 && multilevel(h, F) && (int)F.lv.size() <= mmk::PLEV &&
+         one_launch_rows<T>(h->N) && persistent_smem(h, F) <= PCG_SMEM && lanes_ready(h, F);
 }
 
 // One solve or minimization in flight.  Their number on the device decides how each runs its PCG, so that
@@ -1346,15 +1359,12 @@ void launch_persistent(mm_problem* h, SolverT<TP>& S, SolverT<TV>& F, double tol
   }
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(mmk::PT);
-  const int parts = a.kshift ? (a.G * mmk::WPB) >> a.kshift : 0;  // a block folds its share of these and of b.b's
-  cfg.dynamicSmemBytes = (size_t)((std::max(parts, a.Gdot) + blocks - 1) / blocks) * BS * sizeof(double);
-  if (folded(h, F, 0))  // and keeps its rows of z
-    cfg.dynamicSmemBytes += (size_t)((((a.G * mmk::WPB) >> a.kshift) + blocks - 1) / blocks << a.kshift) * 64 * sizeof(TV);
+  cfg.dynamicSmemBytes = persistent_smem(h, F);
   cfg.stream = h->st;
   cfg.attrs = at;
   cfg.numAttrs = 1;
   auto kern = mmk::k_pcg_persistent<TP, TV>;
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PCG_SMEM));
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   CK(cudaLaunchKernelEx(&cfg, kern, a));
   LAUNCH_CHECK();
