@@ -1584,6 +1584,17 @@ int run_mixed(mm_problem* h, double tol, int maxiter, int* iters, double* r2_out
   return outer;
 }
 
+// whether a kernel of the problem may read and write the vector where it lies (a copy takes any address)
+bool iterable(const mm_problem* h, const double* v) {
+  if (reinterpret_cast<uintptr_t>(v) % sizeof(double) != 0) return false;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, v) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice && at.device == h->device;
+}
+
 // demag solve with the potential in d_U (in/out)
 // h_out (host, or null): the potential is also copied there, behind the solve and inside its one wait.
 // x0_ready (or null): an event the initial guess d_U waits for (its copy from the host on another
@@ -1595,8 +1606,9 @@ int solve_dev(mm_problem* h, const double* d_m, double* d_U, double tol, int max
   const bool mixed = h->mixed && h->s32.built;
   const bool mp = !mixed && h->fp32_precond && h->s32.built && multilevel(h, h->s32);
   // The one-launch PCG takes the caller's U as its iterate and forms b.b itself: two copies and an inner product
-  // less in front of and behind it (10 us of a solve).
-  const bool direct = !mixed && !zero_mean && (mp ? persistent_ok(h, h->s32) && h->use_a0df() : persistent_ok(h, h->s64));
+  // less in front of and behind it (10 us of a solve).  A U that its loads and stores cannot take is copied instead.
+  const bool direct = !mixed && !zero_mean && iterable(h, d_U) &&
+                      (mp ? persistent_ok(h, h->s32) && h->use_a0df() : persistent_ok(h, h->s64));
   CK(cudaEventRecord(h->ev0, h->st));
   enqueue_rhs(h, d_m, !direct);
   if (x0_ready) CK(cudaStreamWaitEvent(h->st, x0_ready, 0));
