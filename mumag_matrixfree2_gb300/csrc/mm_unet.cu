@@ -430,39 +430,57 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad(WgArgs a) {
   }
 }
 
-// (h, l) += v exactly up to the rounding of l
-__device__ __forceinline__ void sum2(float& h, float& l, float v) {
-  const float t = h + v, z = t - h;
-  l += (h - (t - z)) + (v - z);
-  h = t;
-}
+// A sum in three floats: h, the rounding errors of h's sum in m, theirs in l.  What is lost is the rounding of l, 2^-72
+// of the largest partial sum, less than an FP64 sum loses (2^-53).
+struct Sum3 {
+  float h, m, l;
+  static __device__ __forceinline__ float add(float& s, float v) {  // s += v; returns the rounding error (Knuth)
+    const float t = s + v, z = t - s, e = (s - (t - z)) + (v - z);
+    s = t;
+    return e;
+  }
+  __device__ __forceinline__ void add(float v) { l += add(m, add(h, v)); }
+  __device__ __forceinline__ float value() {
+    const float e = add(h, m);
+    return h + (e + l);
+  }
+};
 
 // The gradients from the partials (weights, then biases if any) in a fixed order: 2^lg threads of a block take every
-// 2^lg-th partial of an element each.  Rows ci >= keep_ci of the weights are zeroed.  The sums are FP32 pairs (a sum and
-// its rounding errors, ~2^-47): conversions and adds of FP64 sums held the FP64 pipe for 10-30 us a layer.
+// 2^lg-th partial of an element each.  Rows ci >= keep_ci of the weights are zeroed.  The sums are FP32 triples:
+// conversions and adds of FP64 sums held the FP64 pipe for 10-30 us a layer.  Where FP32's range ends them (a partial that is
+// infinite or NaN, a sum on the way past 3.4e38) an FP64 sum decides.
 __global__ void __launch_bounds__(256) k_sum_parts(const float* part, int nparts, int lg, int nw, int n, int cin,
                                                    int cout, int keep_ci, float* dw, float* db) {
-  __shared__ float2 s[256];
+  __shared__ Sum3 s[256];
   const int per = 256 >> lg, j = threadIdx.x / per;
   const int i = blockIdx.x * per + threadIdx.x % per;
-  float h = 0.0f, l = 0.0f;
+  Sum3 a{};
   if (i < n) {
 #pragma unroll 8
-    for (int k = j; k < nparts; k += 1 << lg) sum2(h, l, part[(size_t)k * n + i]);
+    for (int k = j; k < nparts; k += 1 << lg) a.add(part[(size_t)k * n + i]);
   }
   if (lg) {
-    s[threadIdx.x] = make_float2(h, l);
+    s[threadIdx.x] = a;
     __syncthreads();
     if (j) return;
     for (int k = 1; k < 1 << lg; ++k) {
-      const float2 o = s[threadIdx.x + k * per];
-      sum2(h, l, o.x);
-      l += o.y;
+      const Sum3 o = s[threadIdx.x + k * per];
+      a.add(o.h);
+      a.add(o.m);
+      a.l += o.l;
     }
   }
   if (i >= n) return;
-  if (i >= nw) db[i - nw] = h + l;
-  else dw[i] = (i / cout) % cin < keep_ci ? h + l : 0.0f;
+  float g = a.value();
+  if (!isfinite(g)) {
+    double t = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < nparts; ++k) t += (double)part[(size_t)k * n + i];
+    g = (float)t;
+  }
+  if (i >= nw) db[i - nw] = g;
+  else dw[i] = (i / cout) % cin < keep_ci ? g : 0.0f;
 }
 
 // ------------------------------------------------------------------------------------------------
