@@ -383,9 +383,14 @@ int mm_time_kernel(mm_problem* h, int kernel, int reps, double* ms_per_launch, d
  * (|a_ij| + |a_ji| < 2 eps sqrt(|a_ii a_jj|)) moved into its diagonal, eps in millionths; 0 (default):
  * 0.002; negative: the plain Galerkin operator. */
 #define MM_OPT_SA_FILTER_E6 20
+/* MM_OPT_ONE_LAUNCH: blocks of a demag solve's persistent launch (MM_OPT_GRAPH) at most; each holds an SM until the
+ * solve has converged.  -1 (default): every SM; a third of them beside one or two other solves or minimizations in
+ * flight on the device; no such launch beside more.  0: never such a launch, but separate kernels, between which
+ * other streams' work runs.  The same results either way, bit for bit. */
+#define MM_OPT_ONE_LAUNCH 21
 int mm_set_option(mm_problem* h, int option, int value);
 /* The current value of MM_OPT_COARSE_CYCLE, MM_OPT_FUSE_RESTRICT, MM_OPT_COARSE_FUSE,
- * MM_OPT_ENERGY_FF_LANES or MM_OPT_MIN_GRAPH (after mm_autotune, or after a loop graph that could not
+ * MM_OPT_ENERGY_FF_LANES, MM_OPT_MIN_GRAPH or MM_OPT_ONE_LAUNCH (after mm_autotune, or after a loop graph that could not
  * hold the cooperative launch turned MM_OPT_COARSE_CYCLE off). */
 int mm_get_option(mm_problem* h, int option, int* value);
 

@@ -283,6 +283,7 @@ struct mm_problem {
   mmk::PBar* d_pbar = nullptr;   // the one-launch PCG's grid barrier
   int coop_sms = 0;              // SMs a cooperative launch can fill (0: not supported)
   int pcg_cap = 0;               // blocks of the one-launch PCG at most in this call (SolveScope)
+  int one_launch = -1;           // MM_OPT_ONE_LAUNCH
   mmk::Scalars* d_sc = nullptr;  // scalars of the FP64 solver, the energy and the minimizer
   mmk::Scalars* d_sc32 = nullptr;
   mmk::Scalars* h_sc = nullptr;  // pinned
@@ -1193,12 +1194,15 @@ mmk::POp<T> persistent_op(const DevMatT<T>& M) {
 
 // Blocks: one per 256 rows, at most one per SM (a solve with one per 128, 256, 384 and 512 rows: 59,319 nodes 617,
 // 615, 616 and 664 us, FP32 V-cycle 553, 553, 552 and 583; 45,570 nodes 541, 540, 563 and 602, FP32 482, 483, 483 and
-// 492).  Up to 16 as one cluster of 16, whose hardware barrier costs a quarter of the grid's.
+// 492).  Up to 16 as one cluster of 16, whose hardware barrier costs a quarter of the grid's, if so many are allowed.
 constexpr int PCG_CLUSTER = 16;
 
-int persistent_blocks(mm_problem* h) {
-  const int want = std::min((h->N + 255) / 256, h->pcg_cap);
-  return std::max(want, PCG_CLUSTER);
+bool persistent_cluster(const mm_problem* h) {
+  return h->pcg_cap >= PCG_CLUSTER && (h->N + 255) / 256 <= PCG_CLUSTER;
+}
+
+int persistent_blocks(const mm_problem* h) {
+  return persistent_cluster(h) ? PCG_CLUSTER : std::min(h->pcg_cap, (h->N + 255) / 256);
 }
 
 // Dynamic shared memory of a block: its share of the partials of eight warps and of b.b's, 2 KB each, which it folds, and
@@ -1233,6 +1237,7 @@ struct SolveScope {
   explicit SolveScope(mm_problem* h) : n(g_solving[std::min(std::max(h->device, 0), 63)]) {
     const int k = ++n;
     h->pcg_cap = k == 1 ? h->coop_sms : k <= 3 ? h->coop_sms / 3 : 0;
+    if (h->one_launch >= 0) h->pcg_cap = std::min(h->pcg_cap, h->one_launch);
   }
   ~SolveScope() { --n; }
 };
@@ -1245,7 +1250,7 @@ int persistent_args(mm_problem* h, SolverT<TP>& S, SolverT<TV>& F, mmk::PcgArgs<
   const bool use_rf = (h->fuse_restrict >> bit) & 1;
   const bool fused = F.fused && ((h->coarse_fuse >> bit) & 1);
   const int blocks = persistent_blocks(h);
-  a.cluster = blocks <= PCG_CLUSTER;
+  a.cluster = persistent_cluster(h);
   a.n = h->N;
   a.G = grid_ilp(h->N);
   a.Gdot = std::min(a.G, g_vec_cap);
@@ -4325,6 +4330,7 @@ int mm_get_option(mm_problem* h, int option, int* value) {
     case MM_OPT_COARSE_FUSE: *value = h->coarse_fuse; return MM_OK;
     case MM_OPT_ENERGY_FF_LANES: *value = h->eff_lanes(); return MM_OK;
     case MM_OPT_MIN_GRAPH: *value = h->min_graph; return MM_OK;
+    case MM_OPT_ONE_LAUNCH: *value = h->one_launch; return MM_OK;
     default: return MM_ERR_ARG;
   }
 }
@@ -4463,6 +4469,11 @@ int mm_set_option(mm_problem* h, int option, int value) {
     if (value != 0 && value != 1) return MM_ERR_ARG;
     h->min_graph = value;
     h->min_graph_failed = false;
+    return MM_OK;
+  }
+  if (option == MM_OPT_ONE_LAUNCH) {
+    if (value < -1) return MM_ERR_ARG;
+    h->one_launch = value;  // minimizer graphs are kept by the blocks that follow
     return MM_OK;
   }
   if (option == MM_OPT_MIXED_ETA_E6) {

@@ -9,6 +9,7 @@ import torch
 
 from mumag_matrixfree2_gb300 import _abi, fem_utils
 from mumag_matrixfree2_gb300 import synthetic as syn
+from mumag_matrixfree2_gb300.cuda_backend import MinimizerParams
 
 pytestmark = pytest.mark.gpu
 
@@ -42,3 +43,91 @@ def test_potential_at_any_address(cuda_ok, precision, offset):
     U = np.frombuffer(buf[offset:offset + 8 * s.N].cpu().numpy().tobytes(), np.float64)
     assert np.array_equal(U, ref.cpu().numpy())
     assert not buf[:offset].any() and not buf[offset + 8 * s.N:].any()
+
+
+def _launches(prob, *args):
+    n = prob.launch_count()
+    out = prob.solve_u(*args)
+    return out, prob.launch_count() - n
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_precond", "mixed"])
+@pytest.mark.parametrize("workload", ["cube8_h2_air24", "cube16_h2_air48", "cube40_h2_air200"])
+def test_every_route_of_a_solve_gives_the_same_bits(cuda_ok, workload, precision):
+    """One launch on every SM, on a third of them, on one cluster's number, on fewer blocks than a cluster has; the loop
+    graph of separate kernels; and the host's polling."""
+    s, prob = _problem(workload, precision)
+    m = syn.initial_state(s.N, seed=12, amplitude=0.3)
+    x0 = 0.01 * np.random.default_rng(13).standard_normal(s.N) * s.boundary_mask
+    prob.set_option("graph", 0)
+    ref, polled = _launches(prob, m, x0, 1e-10)
+    prob.set_option("graph", 1)
+    for blocks in (-1, 10**6, 50, 17, 16, 15, 8, 0):
+        prob.set_option("one_launch", blocks)
+        assert prob.get_option("one_launch") == blocks
+        out, n = _launches(prob, m, x0, 1e-10)
+        assert out[1:] == ref[1:] and np.array_equal(out[0], ref[0]), blocks
+        assert (n < polled // 2) == (blocks != 0), (blocks, n, polled)
+    with pytest.raises(_abi.MMError):
+        prob.set_option("one_launch", -2)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_precond", "mixed"])
+def test_loop_graph_holds_the_coarse_cycle(cuda_ok, precision):
+    """The separate kernels' loop graph with levels 1 .. 3 in one cooperative launch, against the one launch: the same
+    bits, fewer launches than with five, and the graph did hold it."""
+    s, prob = _problem("cube80_h1.6_air200", precision)
+    m = syn.initial_state(s.N, seed=14, amplitude=0.1)
+    ref, one = _launches(prob, m, np.zeros(s.N), 1e-10)
+    prob.set_option("one_launch", 0)
+    out, n = [], []
+    for cc in (0, 3):
+        prob.set_option("coarse_cycle", cc)
+        r, k = _launches(prob, m, np.zeros(s.N), 1e-10)
+        assert prob.get_option("coarse_cycle") == cc
+        assert r[1:] == ref[1:] and np.array_equal(r[0], ref[0]), cc
+        n.append(k)
+    assert one < n[1] < n[0]
+
+
+@pytest.mark.parametrize("method,precision,cpp", [("pcohen_hs", "fp64", False), ("pcohen", "fp64", True),
+                                                  ("pcohen_hs", "fp32_precond", False)])
+def test_minimizer_graph_with_every_form_of_its_demag_solve(cuda_ok, method, precision, cpp):
+    """The minimizer's graph with its demag solve as one launch, on a third of the SMs and as a nested loop of separate
+    kernels, against its host loop: the same state, counts and energies."""
+    s, prob = _problem("cube16_h2_air48", precision)
+    m0 = syn.initial_state(s.N, seed=15, amplitude=0.2)
+    mp = MinimizerParams(method=method, max_iter=40, tau_f=1e-8, eps_a=1e-6, cg_tol=1e-10, cpp_semantics=cpp)
+    runs = {}
+    for blocks, graph in ((-1, 1), (50, 1), (0, 1), (-1, 1), (-1, 0), (0, 0)):
+        prob.set_option("one_launch", blocks)
+        prob.set_option("min_graph", graph)
+        m, U, info = prob.minimize(np.array([0.0, 0.0, -0.3]), m0, np.zeros(s.N), mp)
+        assert info["device_loop"] == bool(graph)
+        runs[blocks, graph] = (m, U, [info[k] for k in ("iters", "evals", "preco_iters", "demag_iters", "E", "gnorm")])
+    m, U, counts = runs.pop((0, 0))
+    assert counts[0] > 2
+    for route, r in runs.items():
+        assert r[2] == counts and np.array_equal(r[0], m) and np.array_equal(r[1], U), route
+
+
+def test_a_solve_beside_another_streams_work(cuda_ok):
+    """Kernels of another stream before, beside and after solves of either form: both give what they give alone."""
+    s, prob = _problem("cube40_h2_air200")
+    m = syn.initial_state(s.N, seed=16, amplitude=0.3)
+    ref = prob.solve_u(m, np.zeros(s.N), 1e-10)[0]
+    a = torch.randn(1024, 1024, device="cuda", dtype=torch.float64)
+    want = a
+    for _ in range(8):
+        want = torch.sin(want) + a
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    for blocks in (-1, 50, 0):
+        prob.set_option("one_launch", blocks)
+        with torch.cuda.stream(side):
+            got = a
+            for _ in range(8):
+                got = torch.sin(got) + a
+        U = prob.solve_u(m, np.zeros(s.N), 1e-10)[0]
+        side.synchronize()
+        assert np.array_equal(U, ref) and torch.equal(got, want)
