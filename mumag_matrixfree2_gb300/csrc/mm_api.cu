@@ -1224,22 +1224,28 @@ bool persistent_ok(mm_problem* h, SolverT<T>& F) {
          one_launch_rows<T>(h->N) && persistent_smem(h, F) <= PCG_SMEM && lanes_ready(h, F);
 }
 
-// One solve or minimization in flight.  Their number on the device decides how each runs its PCG, so that
+// One solve, minimization or autotuning in flight.  Their number on the device decides how each runs its PCG, so that
 // several threads' problems share the GPU: alone on every SM, with one or two others on a third of them each,
 // and with more as separate kernels, whose many small launches overlap (48 particles on 16 threads, FP32
 // V-cycle: 16.3 s with every SM for each, 13.2 s with a cluster of 16 blocks each, 11.1 s as separate kernels, now
-// 10.2).
+// 10.2).  The cap holds for the call: outside one there is none to use.
 // The results are the same bits.
 std::atomic<int> g_solving[64];
 
 struct SolveScope {
+  mm_problem* const h;
   std::atomic<int>& n;
-  explicit SolveScope(mm_problem* h) : n(g_solving[std::min(std::max(h->device, 0), 63)]) {
+  explicit SolveScope(mm_problem* p) : h(p), n(g_solving[std::min(std::max(p->device, 0), 63)]) {
     const int k = ++n;
     h->pcg_cap = k == 1 ? h->coop_sms : k <= 3 ? h->coop_sms / 3 : 0;
     if (h->one_launch >= 0) h->pcg_cap = std::min(h->pcg_cap, h->one_launch);
   }
-  ~SolveScope() { --n; }
+  ~SolveScope() {
+    h->pcg_cap = 0;
+    --n;
+  }
+  SolveScope(const SolveScope&) = delete;
+  SolveScope& operator=(const SolveScope&) = delete;
 };
 
 // The arguments of the one-launch PCG; returns its blocks.
@@ -3540,7 +3546,7 @@ int mm_create(int N, int E, const int* conn, const double* volume, const double*
       if (sms > 0) g_vec_cap = std::min(4 * sms, MAXG);
       int coop = 0;
       CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-      h->coop_sms = h->pcg_cap = coop ? sms : 0;
+      h->coop_sms = coop ? sms : 0;
     }
     CK(cudaEventCreate(&h->ev0));
     CK(cudaEventCreate(&h->ev1));
@@ -4296,6 +4302,7 @@ int mm_autotune(mm_problem* h, int reps, char* report, int report_len) {
   if (!h || reps < 1) return MM_ERR_ARG;
   return guarded(h, [&] {
     if (!h->poisson_built) throw Fail{MM_ERR_STATE, "mm_build_poisson must be called first"};
+    SolveScope in_flight(h);
     std::string ops = "[";
     tune_solver<double>(h, h->s64, reps, ops);
     tune_solver<float>(h, h->s32, reps, ops);

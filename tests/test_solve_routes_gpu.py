@@ -2,6 +2,7 @@
 change: the potential, the calls that are taken, and what a handle keeps from one call for the next."""
 
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -131,3 +132,41 @@ def test_a_solve_beside_another_streams_work(cuda_ok):
         U = prob.solve_u(m, np.zeros(s.N), 1e-10)[0]
         side.synchronize()
         assert np.array_equal(U, ref) and torch.equal(got, want)
+
+
+def test_autotuner_does_not_depend_on_the_last_call(cuda_ok):
+    """A solve beside three other problems' runs as separate kernels; the autotuner of that handle, called alone later, times
+    the one launch all the same: about as many launches as on a handle that never had company."""
+    s, prob = _problem("cube16_h2_air48")
+    m = syn.initial_state(s.N, seed=17, amplitude=0.3)
+    others = [_problem("cube8_h2_air24") for _ in range(3)]
+    zero = np.zeros(s.N)
+    alone = _launches(prob, m, zero, 1e-10)[1]
+    stop = threading.Event()
+    gate = threading.Barrier(4)
+
+    def work(so, po):
+        mo = syn.initial_state(so.N, seed=18, amplitude=0.3)
+        gate.wait()
+        while not stop.is_set():
+            po.minimize(np.array([0.0, 0.0, -0.3]), mo, np.zeros(so.N), MinimizerParams(max_iter=40, tau_f=1e-12))
+
+    threads = [threading.Thread(target=work, args=o) for o in others]
+    for t in threads:
+        t.start()
+    gate.wait()
+    beside = []
+    for _ in range(2000):
+        beside.append(_launches(prob, m, zero, 1e-10)[1])
+        if beside[-1] > 4 * alone:
+            break
+    stop.set()
+    for t in threads:
+        t.join()
+    assert beside[-1] > 4 * alone  # the handle's last solve ran as separate kernels
+    counts = []
+    for p in (prob, _problem("cube16_h2_air48")[1]):
+        n = p.launch_count()
+        p.autotune(reps=3)
+        counts.append(p.launch_count() - n)
+    assert counts[0] <= 1.25 * counts[1], counts
