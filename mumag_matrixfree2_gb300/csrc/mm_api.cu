@@ -399,6 +399,15 @@ struct mm_problem {
     CK(cudaMemsetAsync(p, 0, n * sizeof(T), st));
     return (T*)p;
   }
+  // gives a buffer back behind the work queued on the stream (never while it captures)
+  template <class T>
+  void release(const T*& p) {
+    const auto at = std::find(allocs.begin(), allocs.end(), (void*)p);
+    if (at == allocs.end()) return;
+    CK(cudaFreeAsync(*at, st));
+    allocs.erase(at);
+    p = nullptr;
+  }
   template <class T, class Alloc>
   T* upload(const std::vector<T, Alloc>& v) {
     T* p = alloc<T>(v.size());
@@ -845,6 +854,27 @@ void ensure_lanes(mm_problem* h, SolverT<T>& S) {
   for (int l = 0; l < (int)S.lv.size() - 1; ++l)
     level_operators(h, S, l, [&](DevMatT<T>& M, const mm::HostCSR& host, const char*) { h->upload_lanes<T>(host, M); },
                     [](DevMatT<T>&, const mm::HostCSR&, const char*) {});
+}
+
+// Gives back the layouts that no solve reads now: those for other numbers of lanes than the operator's, and those of the
+// one-launch PCG of operators that its V-cycle does not read.  The graphs that hold them have been dropped.
+template <class T>
+void trim_lanes(mm_problem* h, SolverT<T>& S) {
+  auto drop = [h](mmk::SellT<T>& o) {
+    if (!o.sptr) return;
+    h->release(o.sptr);
+    h->release(o.col);
+    h->release(o.val);
+    o = mmk::SellT<T>{};
+  };
+  auto keep = [&](DevMatT<T>& M, int tpr) {
+    if (M.c.n > 0 && M.tpr != 1) drop(M.s);
+    for (int lg = 1; lg <= 5; ++lg)
+      if ((1 << lg) != tpr) drop(M.lanes[lg - 1]);
+  };
+  for (int l = 0; l < (int)S.lv.size() - 1; ++l)
+    level_operators(h, S, l, [&](DevMatT<T>& M, const mm::HostCSR&, const char*) { keep(M, M.tpr); },
+                    [&](DevMatT<T>& M, const mm::HostCSR&, const char*) { keep(M, 0); });
 }
 
 template <class T>
@@ -4311,6 +4341,10 @@ int mm_autotune(mm_problem* h, int reps, char* report, int report_len) {
     const std::string f32 = tune_fuse<float>(h, h->s32, 1, reps);
     const std::string r64 = tune_fuse_restrict<double>(h, h->s64, 0, reps);
     const std::string r32 = tune_fuse_restrict<float>(h, h->s32, 1, reps);
+    ensure_lanes(h, h->s64);
+    ensure_lanes(h, h->s32);
+    trim_lanes(h, h->s64);
+    trim_lanes(h, h->s32);
     const std::string eff = tune_energy_ff(h, reps);
     const std::string c64 = tune_coarse_cycle<double>(h, h->s64, 0, reps);
     const std::string c32 = tune_coarse_cycle<float>(h, h->s32, 1, reps);
@@ -4450,6 +4484,7 @@ int mm_set_option(mm_problem* h, int option, int value) {
         }
         ensure_lanes(h, S);
         drop_graph(S);
+        trim_lanes(h, S);
       };
       set_all(h->s64);
       set_all(h->s32);

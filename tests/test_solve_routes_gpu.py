@@ -170,3 +170,39 @@ def test_autotuner_does_not_depend_on_the_last_call(cuda_ok):
         p.autotune(reps=3)
         counts.append(p.launch_count() - n)
     assert counts[0] <= 1.25 * counts[1], counts
+
+
+def _pool_bytes():
+    """Bytes in use of the device's default memory pool, which holds every problem's buffers."""
+    cu = C.CDLL("libcuda.so.1")
+    pool, used = C.c_void_p(), C.c_uint64()
+    torch.cuda.synchronize()
+    assert cu.cuDeviceGetDefaultMemPool(C.byref(pool), torch.cuda.current_device()) == 0
+    assert cu.cuMemPoolGetAttribute(pool, 7, C.byref(used)) == 0  # CU_MEMPOOL_ATTR_USED_MEM_CURRENT
+    return used.value
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_precond", "mixed"])
+def test_autotuner_keeps_one_layout_of_an_operator(cuda_ok, precision):
+    """Neither autotuning nor setting the lanes leaves a copy of an operator for every number of lanes that was tried:
+    at most a second one where the lanes that are kept need more padding."""
+    s, prob = _problem("cube40_h2_air200", precision)
+    m = syn.initial_state(s.N, seed=19, amplitude=0.3)
+    ref = prob.solve_u(m, np.zeros(s.N), 1e-10)
+    before = _pool_bytes()
+    for lanes in (2, 4, 8, 16, 32, 8):
+        prob.set_option("csr_lanes", lanes)
+        prob.solve_u(m, np.zeros(s.N), 1e-10)
+    entry = {"fp64": 12, "fp32": 8}
+    rep = prob.autotune(reps=2)
+    once = sum(o["nnz"] * entry[o["precision"]] for o in rep["operators"])
+    assert _pool_bytes() - before <= 2 * once
+    for _ in range(2):
+        prob.autotune(reps=1)
+    assert _pool_bytes() - before <= 2 * once
+    for restrict, coarse in ((0, 0), (3, 3)):  # operators laid out anew where they come into use again
+        prob.set_option("fuse_restrict", restrict)
+        prob.set_option("coarse_fuse", coarse)
+        out, n = _launches(prob, m, np.zeros(s.N), 1e-10)
+        assert n < 8 * max(1, prob.last_refinements()) and abs(out[1] - ref[1]) <= (2 if precision == "mixed" else 1)
+        assert np.abs(out[0] - ref[0]).max() <= 1e-7 * np.abs(ref[0]).max()
