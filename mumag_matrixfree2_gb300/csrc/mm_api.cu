@@ -281,7 +281,8 @@ struct mm_problem {
   float *d_r32 = nullptr, *d_d32 = nullptr;
   double* d_part = nullptr;      // NRED x MAXG block partials (shared by every reduction)
   mmk::PBar* d_pbar = nullptr;   // the one-launch PCG's grid barrier
-  int coop_sms = 0;              // SMs a cooperative launch can fill (0: not supported)
+  int coop_sms = 0;              // blocks of the one-launch PCG that the device can hold at once
+  bool pcg_clusters = false;     // and whether a cluster of them
   int pcg_cap = 0;               // blocks of the one-launch PCG at most in this call (SolveScope)
   int one_launch = -1;           // MM_OPT_ONE_LAUNCH
   mmk::Scalars* d_sc = nullptr;  // scalars of the FP64 solver, the energy and the minimizer
@@ -1228,7 +1229,7 @@ mmk::POp<T> persistent_op(const DevMatT<T>& M) {
 constexpr int PCG_CLUSTER = 16;
 
 bool persistent_cluster(const mm_problem* h) {
-  return h->pcg_cap >= PCG_CLUSTER && (h->N + 255) / 256 <= PCG_CLUSTER;
+  return h->pcg_clusters && h->pcg_cap >= PCG_CLUSTER && (h->N + 255) / 256 <= PCG_CLUSTER;
 }
 
 int persistent_blocks(const mm_problem* h) {
@@ -1238,6 +1239,46 @@ int persistent_blocks(const mm_problem* h) {
 // Dynamic shared memory of a block: its share of the partials of eight warps and of b.b's, 2 KB each, which it folds, and
 // with level 0 folded its rows of z.  The largest: 4096 partials (2.1M rows and more) over a third of the SMs, 164 KB.
 constexpr size_t PCG_SMEM = 200 * 1024;
+
+template <class TP, class TV>
+cudaLaunchConfig_t persistent_config(int blocks, bool cluster, size_t smem, cudaStream_t st, cudaLaunchAttribute* at) {
+  if (cluster) {
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = blocks;
+    at->val.clusterDim.y = 1;
+    at->val.clusterDim.z = 1;
+  } else {
+    at->id = cudaLaunchAttributeCooperative;
+    at->val.cooperative = 1;
+  }
+  CK(cudaFuncSetAttribute(mmk::k_pcg_persistent<TP, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PCG_SMEM));
+  CK(cudaFuncSetAttribute(mmk::k_pcg_persistent<TP, TV>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(mmk::PT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// What the device can hold of the launch, with the most shared memory that one takes: blocks of a cooperative grid, and
+// whether a cluster of 16 finds room (a partition of the device may have no 16 SMs side by side).  What it cannot is not
+// tried: a grid in a cluster's place, and separate kernels in a grid's.
+template <class TP, class TV>
+void persistent_room(int sms, int& blocks, bool& clusters) {
+  cudaLaunchAttribute at;
+  int per_sm = 0, n = 0;
+  const cudaLaunchConfig_t cfg = persistent_config<TP, TV>(PCG_CLUSTER, true, PCG_SMEM, nullptr, &at);
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mmk::k_pcg_persistent<TP, TV>, mmk::PT, PCG_SMEM));
+  blocks = std::min(blocks, per_sm * sms);
+  if (cudaOccupancyMaxActiveClusters(&n, mmk::k_pcg_persistent<TP, TV>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  clusters = clusters && n > 0;
+}
 
 template <class T>
 size_t persistent_smem(mm_problem* h, const SolverT<T>& F) {
@@ -1387,27 +1428,9 @@ void launch_persistent(mm_problem* h, SolverT<TP>& S, SolverT<TV>& F, double tol
   const int blocks = persistent_args(h, S, F, a);
   a.tol = tol;
   a.maxiter = maxiter;
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
-  if (a.cluster) {
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = blocks;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-  } else {
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-  }
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(mmk::PT);
-  cfg.dynamicSmemBytes = persistent_smem(h, F);
-  cfg.stream = h->st;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  auto kern = mmk::k_pcg_persistent<TP, TV>;
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PCG_SMEM));
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  CK(cudaLaunchKernelEx(&cfg, kern, a));
+  cudaLaunchAttribute at;
+  const cudaLaunchConfig_t cfg = persistent_config<TP, TV>(blocks, a.cluster != 0, persistent_smem(h, F), h->st, &at);
+  CK(cudaLaunchKernelEx(&cfg, mmk::k_pcg_persistent<TP, TV>, a));
   LAUNCH_CHECK();
 }
 
@@ -3574,9 +3597,6 @@ int mm_create(int N, int E, const int* conn, const double* volume, const double*
       CK(cudaGetDevice(&dev));
       CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
       if (sms > 0) g_vec_cap = std::min(4 * sms, MAXG);
-      int coop = 0;
-      CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-      h->coop_sms = coop ? sms : 0;
     }
     CK(cudaEventCreate(&h->ev0));
     CK(cudaEventCreate(&h->ev1));
@@ -3721,6 +3741,19 @@ int mm_build_poisson(mm_problem* h, double reg, int precond_type, int max_levels
       h->s32.b = h->d_r32;
       h->s32.x = h->d_d32;
       h->s32.sc = h->d_sc32;
+    }
+    if (amg) {
+      int sms = 0, coop = 0;
+      CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+      CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device));
+      h->coop_sms = coop ? sms : 0;
+      h->pcg_clusters = coop != 0;
+      if (h->mixed) {
+        persistent_room<float, float>(sms, h->coop_sms, h->pcg_clusters);
+      } else {
+        persistent_room<double, double>(sms, h->coop_sms, h->pcg_clusters);
+        if (h->fp32_precond) persistent_room<double, float>(sms, h->coop_sms, h->pcg_clusters);
+      }
     }
     h->sync();
     h->poisson_built = true;

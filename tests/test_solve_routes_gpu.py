@@ -2,7 +2,12 @@
 change: the potential, the calls that are taken, and what a handle keeps from one call for the next."""
 
 import ctypes as C
+import json
+import os
+import subprocess
+import sys
 import threading
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -206,3 +211,60 @@ def test_autotuner_keeps_one_layout_of_an_operator(cuda_ok, precision):
         out, n = _launches(prob, m, np.zeros(s.N), 1e-10)
         assert n < 8 * max(1, prob.last_refinements()) and abs(out[1] - ref[1]) <= (2 if precision == "mixed" else 1)
         assert np.abs(out[0] - ref[0]).max() <= 1e-7 * np.abs(ref[0]).max()
+
+
+# a runtime whose occupancy queries say that the device holds no cluster of 16, or no block, of a kernel with 200 KB
+NO_ROOM = """
+#include <dlfcn.h>
+#include <stddef.h>
+#include <stdlib.h>
+int cudaOccupancyMaxActiveClusters(int* n, const void* f, const void* cfg) { *n = 0; return 0; }
+int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* f, int t, size_t smem, unsigned fl) {
+  void* rt = dlopen("libcudart.so.13", RTLD_NOLOAD | RTLD_LAZY);
+  int (*real)(int*, const void*, int, size_t, unsigned) =
+      rt ? dlsym(rt, "cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags") : NULL;
+  int rc = real ? real(n, f, t, smem, fl) : 1;
+  if (getenv("NO_BLOCKS") && smem == 200 * 1024) *n = 0;
+  return rc;
+}
+"""
+
+
+def _solve_small(precision):
+    s, prob = _problem(precision=precision)
+    (U, it, rr, rc), n = _launches(prob, syn.initial_state(s.N, seed=20, amplitude=0.3), np.zeros(s.N), 1e-10)
+    return {"U": [float(u).hex() for u in U], "it": it, "rr": rr.hex(), "rc": rc, "launches": n}
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_precond", "mixed"])
+def test_a_device_without_room_for_the_launch(cuda_ok, precision, tmp_path):
+    """A device that cannot place the cluster runs a grid of blocks, one that cannot place a block separate kernels: the
+    same potential, and no failed launch.  What the runtime says is faked in a process of its own."""
+    (tmp_path / "fake.c").write_text(NO_ROOM)
+    fake = tmp_path / "fake.so"
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(fake), str(tmp_path / "fake.c"), "-ldl"], check=True)
+    ref = _solve_small(precision)
+    root = Path(__file__).resolve().parents[1]
+    code = f"import json; from tests.test_solve_routes_gpu import _solve_small; print(json.dumps(_solve_small({precision!r})))"
+    for env in ({}, {"NO_BLOCKS": "1"}):
+        r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300,
+                           env={**os.environ, "LD_PRELOAD": str(fake), **env})
+        assert r.returncode == 0, r.stderr[-2000:]
+        got = json.loads(r.stdout.strip().splitlines()[-1])
+        n, n0 = got.pop("launches"), ref["launches"]
+        assert got == {k: v for k, v in ref.items() if k != "launches"}
+        assert (n > 2 * n0) if env else (n == n0), (n, n0)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_precond"])
+def test_few_blocks_for_many_rows(cuda_ok, precision):
+    """357,911 rows: eight blocks hold their 88 partials of 2 KB each in shared memory; four cannot, and the solve takes the
+    separate kernels."""
+    s, prob = _problem("cube80_h1.6_air200", precision)
+    m = syn.initial_state(s.N, seed=21, amplitude=0.3)
+    ref, one = _launches(prob, m, np.zeros(s.N), 1e-10)
+    for blocks in (8, 4):
+        prob.set_option("one_launch", blocks)
+        out, n = _launches(prob, m, np.zeros(s.N), 1e-10)
+        assert out[1:] == ref[1:] and np.array_equal(out[0], ref[0]), blocks
+        assert (n == one) == (blocks == 8)
