@@ -823,7 +823,8 @@ bool folded(const mm_problem* h, const SolverT<T>& S, int l) {
   const int bit = sizeof(T) == 8 ? 0 : 1;
   return ((h->fuse_restrict >> bit) & 1) && S.lv[l].G.nnz > 0 && S.lv[l].Rf.nnz > 0 &&
          l < (S.fused && ((h->coarse_fuse >> bit) & 1) ? L - 2 : L - 1) &&
-         (l > 0 || (int64_t)grid_ilp(h->N) * mmk::CHUNK >= h->N);  // pfold0 makes one round of the grid's blocks
+         // pfold0: partials of one warp, and one round of the grid's blocks
+         (l > 0 || (red_kshift(h->N) == 0 && (int64_t)grid_ilp(h->N) * mmk::CHUNK >= h->N));
 }
 
 // f(operator, host copy, name) for the operators of level l below the coarsest that a V-cycle reads (level 0's A,
@@ -1236,8 +1237,8 @@ int persistent_blocks(const mm_problem* h) {
   return persistent_cluster(h) ? PCG_CLUSTER : std::min(h->pcg_cap, (h->N + 255) / 256);
 }
 
-// Dynamic shared memory of a block: its share of the partials of eight warps and of b.b's, 2 KB each, which it folds, and
-// with level 0 folded its rows of z.  The largest: 4096 partials (2.1M rows and more) over a third of the SMs, 164 KB.
+// Dynamic shared memory of a block: its share of the partials of eight warps or of b.b's, 2 KB each, which it folds, or,
+// with level 0 folded, its rows of z.  The largest: 4096 partials (2.1M rows and more) over a third of the SMs, 164 KB.
 constexpr size_t PCG_SMEM = 200 * 1024;
 
 template <class TP, class TV>
@@ -1285,7 +1286,7 @@ size_t persistent_smem(mm_problem* h, const SolverT<T>& F) {
   const int blocks = persistent_blocks(h), G = grid_ilp(h->N), kshift = red_kshift(h->N);
   const int parts = (G * mmk::WPB) >> kshift, dots = std::min(G, g_vec_cap);
   size_t bytes = (size_t)((std::max(kshift ? parts : 0, dots) + blocks - 1) / blocks) * BS * sizeof(double);
-  if (folded(h, F, 0)) bytes += (size_t)((parts + blocks - 1) / blocks << kshift) * 64 * sizeof(T);
+  if (folded(h, F, 0)) bytes = std::max(bytes, (size_t)((parts + blocks - 1) / blocks) * 64 * sizeof(T));
   return bytes;
 }
 

@@ -532,22 +532,22 @@ __device__ __forceinline__ void preduce(const PcgArgs<TP, TV>& a, int kind, PSca
 }
 
 // The folded prolongation on level 0, z = A [r; e] (e behind r in memory), and r.z.  The rows may be dealt out over lanes
-// (below 16Ki rows), and a block takes those of its partials, whose
-// sums it then forms in k_rz's order from shared memory.  Small problems only, so a unit is 64 rows (no second round
-// of a grid's blocks).
+// (below 16Ki rows), and a block takes those of its partials, whose sums it then forms in k_rz's order from shared
+// memory.  Small problems only (folded()): a partial is one warp's unit of 64 rows, with no second round of a grid's
+// blocks.
 template <class TP, class TV>
 __device__ __forceinline__ void pfold0(const PcgArgs<TP, TV>& a, const PStep<TV>& st, int c0, int nc) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const POp<TV> A = st.A;
-  const int n = A.n, lg = A.lg, kshift = a.kshift, U = nc << kshift;
+  const int n = A.n, lg = A.lg;
   double* const pa = a.part + (size_t)R_RZ * MAXG + c0;
-  TV* const s_z = reinterpret_cast<TV*>(s_unit + (kshift ? 32 * U : 0));
+  TV* const s_z = reinterpret_cast<TV*>(s_unit);
   auto row0 = [&](int u, int q) {
-    const int ug = (c0 << kshift) + u;
+    const int ug = c0 + u;
     return ug / WPB * CHUNK + 32 * (ug % WPB) + q * BS;
   };
 #pragma unroll 1
-  for (int k = wid; k < U << (lg + 1); k += PW) {
+  for (int k = wid; k < nc << (lg + 1); k += PW) {
     const int g = k >> lg, sub = k & ((1 << lg) - 1), r0 = row0(g >> 1, g & 1) + (sub << (5 - lg));
     if (r0 >= n) continue;
     const TV ax = planes<TV>(A, st.x, r0 >> (5 - lg));
@@ -560,19 +560,18 @@ __device__ __forceinline__ void pfold0(const PcgArgs<TP, TV>& a, const PStep<TV>
   TV r[2] = {};  // the first unit's, in flight over the barrier
 #pragma unroll
   for (int q = 0; q < 2; ++q)
-    if (wid < U && row0(wid, q) + lane < n) r[q] = st.x[row0(wid, q) + lane];
+    if (wid < nc && row0(wid, q) + lane < n) r[q] = st.x[row0(wid, q) + lane];
   __syncthreads();
 #pragma unroll 1
-  for (int u = wid; u < U; u += PW) {
+  for (int u = wid; u < nc; u += PW) {
     Acc<TV> acc;
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       const int i = row0(u, q) + lane;
       if (i < n) acc.add(u == wid ? r[q] : st.x[i], s_z[64 * u + 32 * q + lane]);
     }
-    punit_out(acc, pa, kshift, u);
+    punit_out(acc, pa, 0, u);
   }
-  pparts_out<TV>(pa, kshift, nc);
 }
 
 // b.b -> R_BB with k_dot's blocks (a partial of eight warps each)
