@@ -383,6 +383,16 @@ struct mm_problem {
   // problems have queued on the device, so problems can be created and destroyed while others run.
   template <class T>
   T* alloc(size_t n) {
+    T* const p = take<T>(n);
+    // zeroed: reused device memory can hold any bit pattern (a NaN in an FP32 view of old FP64 data),
+    // and a vector read once with a zero factor (the first direction's beta p) must not carry it in.
+    // On the problem's own stream, ahead of any copy into the buffer (that stream does not order with
+    // the legacy default stream).
+    CK(cudaMemsetAsync(p, 0, std::max<size_t>(n, 1) * sizeof(T), st));
+    return p;
+  }
+  template <class T>
+  T* take(size_t n) {
     void* p = nullptr;
     if (n == 0) n = 1;
     if (!st) throw Fail{MM_ERR_CUDA, "device allocation before the problem's stream exists"};
@@ -393,11 +403,6 @@ struct mm_problem {
     if (cap != cudaStreamCaptureStatusNone) throw Fail{MM_ERR_STATE, "device allocation while the stream captures"};
     CK(cudaMallocAsync(&p, n * sizeof(T), st));
     allocs.push_back(p);
-    // zeroed: reused device memory can hold any bit pattern (a NaN in an FP32 view of old FP64 data),
-    // and a vector read once with a zero factor (the first direction's beta p) must not carry it in.
-    // On the problem's own stream, ahead of any copy into the buffer (that stream does not order with
-    // the legacy default stream).
-    CK(cudaMemsetAsync(p, 0, n * sizeof(T), st));
     return (T*)p;
   }
   // gives a buffer back behind the work queued on the stream (never while it captures)
@@ -411,8 +416,9 @@ struct mm_problem {
   }
   template <class T, class Alloc>
   T* upload(const std::vector<T, Alloc>& v) {
-    T* p = alloc<T>(v.size());
-    if (!v.empty()) CK(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st));
+    if (v.empty()) return alloc<T>(0);
+    T* const p = take<T>(v.size());  // all of it is written here
+    CK(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st));
     return p;
   }
   template <class T, class Alloc>
@@ -612,7 +618,7 @@ struct mm_problem {
     }
     std::vector<int> col(sptr[ns], 0);
     std::vector<T> val(sptr[ns], T(0));
-    mm::parallel_rows(A.n_rows, sptr[ns], [&](int64_t r0, int64_t r1) {
+    mm::parallel_rows(A.n_rows, sptr[ns] / 4, [&](int64_t r0, int64_t r1) {
       for (int r = (int)r0; r < (int)r1; ++r) {
         const int s = r / per, w2 = (sptr[s + 1] - sptr[s]) / 32, len = A.ptr[r + 1] - A.ptr[r];
         if (len == 0) continue;
@@ -3337,7 +3343,7 @@ void build_solver(mm_problem* h, SolverT<T>& S, const mm::HostCSR& A, bool amg, 
         std::vector<double> sd(hl.A.n_rows);
         for (int i = 0; i < hl.A.n_rows; ++i)
           sd[i] = precond_type == MM_PRECOND_AMGCL ? hl.spai0[i] : 0.6667 / (hl.diag[i] + 1e-30);
-        g = mm::folded_prolongation(hl.A, hl.P, sd, fold_offset(hl.A.n_rows));
+        g = mm::folded_prolongation(hl.A, h->rf_host[l], sd, fold_offset(hl.A.n_rows));
       }
       // level 0 from 16Ki rows on by one thread a row: 59,319 rows, a V-cycle with 1, 2, 4 and 8 lanes 38.4, 39.0,
       // 39.2 and 40.1 us

@@ -132,8 +132,9 @@ HostCSR fused_restriction(const HostCSR& R, const HostCSR& A, const std::vector<
 // the same from the product RA = R A: R - (R A) S, with no second sparse product
 HostCSR fused_restriction_ra(const HostCSR& R, const HostCSR& RA, const std::vector<double>& s);
 // G = [2S - S A S | (I - S A) P], S = diag(s): from a level's right-hand side and the coarse correction, stacked with
-// the latter from row `offset` on, to the post-smoothed iterate
-HostCSR folded_prolongation(const HostCSR& A, const HostCSR& P, const std::vector<double>& s, int offset);
+// the latter from row `offset` on, to the post-smoothed iterate.  A is symmetric and R = P^T, so (I - S A) P is the
+// transpose of the fused restriction Rf = R (I - A S), and costs no sparse product.
+HostCSR folded_prolongation(const HostCSR& A, const HostCSR& Rf, const std::vector<double>& s, int offset);
 // f(begin, end) on chunks of [0, n) by the setup's host threads (`work`: its items, for their number)
 void parallel_rows(int64_t n, int64_t work, const std::function<void(int64_t, int64_t)>& f);
 std::vector<double> dense_inverse(const HostCSR& A);  // row-major n x n; throws on singular
