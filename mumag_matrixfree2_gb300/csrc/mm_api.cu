@@ -86,7 +86,7 @@ template <class T>
 struct DevMatT {
   mmk::SellT<T> s{};
   mmk::CsrT<T> c{};
-  mmk::SellT<T> lanes[5]{};  // the rows dealt out over 2, 4 .. 32 lanes, for the one-launch PCG (upload_lanes)
+  mmk::SellT<T> lanes[5]{};  // the rows dealt out over 2, 4 .. 32 lanes (upload_lanes)
   int tpr = 1;
   int64_t nnz = 0;     // stored non-zeros (without padding)
   int64_t stored = 0;  // entries including padding
@@ -597,7 +597,7 @@ struct mm_problem {
     upload_sell<T>(A, d);
     return d;
   }
-  // What the one-launch PCG reads of an operator with tpr > 1: its rows dealt out over tpr lanes (entry k to lane
+  // What the one-launch PCG, and the separate kernels, read of an operator with tpr > 1: its rows dealt out over tpr lanes (entry k to lane
   // k % tpr) and the lanes laid out as the rows of a sliced ELL, so that a warp's loads of columns and values are
   // contiguous.  Read from the compressed rows, 16 rows by two lanes each are 16 separate pieces to a load, and the
   // L1's wavefronts took half of a restriction's time.  FP64 solves from compressed and from dealt-out rows:
@@ -769,10 +769,20 @@ void launch(mm_problem* h, void (*kern)(KArgs...), dim3 grid, dim3 block, Args..
     default: { constexpr int TP = 32; __VA_ARGS__; } break; \
   }
 
+// the rows of an operator dealt out over its lanes (upload_lanes), null where it has none such
+template <class T>
+const mmk::SellT<T>* dealt_rows(const DevMatT<T>& M) {
+  int lg = 0;
+  while ((1 << lg) < M.tpr) ++lg;
+  return lg > 0 && M.lanes[lg - 1].sptr ? &M.lanes[lg - 1] : nullptr;
+}
+
 template <int MODE, class T>
 void spmv(mm_problem* h, const DevMatT<T>& A, const T* x, const T* b, const T* s, T* y, const int* done) {
   if (A.tpr == 1) {
     launch(h, mmk::k_sell<MODE, T>, grid_ilp(A.s.n), BS, A.s, x, b, s, y, done);
+  } else if (const mmk::SellT<T>* o = dealt_rows(A)) {
+    launch(h, mmk::k_dealt<MODE, T>, grid_rows(o->n, A.tpr), BS, *o, A.tpr, x, b, s, y, (T*)nullptr, done);
   } else {
     const int g = grid_rows(A.c.n, A.tpr);
     TPR_SWITCH(A.tpr, (launch(h, mmk::k_csr<TP, MODE, T>, g, BS, A.c, x, b, s, y, done)));
@@ -922,6 +932,9 @@ void enqueue_vcycle(mm_problem* h, SolverT<T>& S, const T* r, T* z, bool in_loop
     tagged<T>(h, MM_PROF_RESTRICT, l, rbytes, [&] {
       if (M.tpr == 1) {
         launch(h, mmk::k_restrict<T>, grid_ilp(nx.n), BS, M.s, in, nx.b, no_pre ? nullptr : nx.s, nx.x, done);
+      } else if (const mmk::SellT<T>* o = dealt_rows(M)) {
+        launch(h, mmk::k_dealt<4, T>, grid_rows(o->n, M.tpr), BS, *o, M.tpr, in, (const T*)nullptr,
+               no_pre ? nullptr : nx.s, nx.b, nx.x, done);
       } else {
         const int g = grid_rows(nx.n, M.tpr);
         TPR_SWITCH(M.tpr, (launch(h, mmk::k_restrict_csr<TP, T>, g, BS, M.c, in, nx.b, no_pre ? nullptr : nx.s,

@@ -268,3 +268,22 @@ def test_few_blocks_for_many_rows(cuda_ok, precision):
         out, n = _launches(prob, m, np.zeros(s.N), 1e-10)
         assert out[1:] == ref[1:] and np.array_equal(out[0], ref[0]), blocks
         assert (n == one) == (blocks == 8)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_precond"])
+def test_dealt_out_rows_against_compressed_rows(cuda_ok, precision):
+    """The separate kernels read rows dealt out over their lanes; the coarse cycle reads the same operators' compressed rows
+    (level 1, folded and not): for every number of lanes the same solve bit for bit, in the loop graph and polled."""
+    s, prob = _problem("cube80_h1.6_air200", precision)
+    m = syn.initial_state(s.N, seed=22, amplitude=0.3)
+    prob.set_option("one_launch", 0)
+    for lanes in (2, 4, 8, 16, 32):
+        prob.set_option("csr_lanes", lanes)
+        ref = None
+        for graph, cycle in ((1, 0), (1, 3), (0, 3), (0, 0)):
+            prob.set_option("graph", graph)
+            prob.set_option("coarse_cycle", cycle)
+            out = prob.solve_u(m, np.zeros(s.N), 1e-10)
+            assert prob.get_option("coarse_cycle") == cycle and out[3] == 0
+            ref = ref or out
+            assert out[1:] == ref[1:] and np.array_equal(out[0], ref[0]), (lanes, graph, cycle)
