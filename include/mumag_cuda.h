@@ -283,8 +283,8 @@ int mm_minimize_dev(mm_problem* h, const double* B_ext, double* d_m_inout, doubl
 int mm_time_kernel(mm_problem* h, int kernel, int reps, double* ms_per_launch, double* bytes_per_launch);
 
 /* Solver options.  MM_OPT_GRAPH (default 1): run a demag solve on the device until convergence: as one
- * persistent launch (multilevel preconditioners; FP32 V-cycles up to 786,432 nodes; fewer than four solves or
- * minimizations in flight on the device), else as separate kernels inside a CUDA graph whose conditional WHILE
+ * persistent launch (multilevel preconditioners; FP32 V-cycles up to 786,432 nodes and, as the preconditioner of the
+ * FP64 PCG, with MM_OPT_SPLIT_A0; MM_OPT_ONE_LAUNCH), else as separate kernels inside a CUDA graph whose conditional WHILE
  * node loops; 0 polls the device flag from the host every four iterations (separate kernels).  The same
  * results either way, bit for bit. */
 #define MM_OPT_GRAPH 1
@@ -384,8 +384,8 @@ int mm_time_kernel(mm_problem* h, int kernel, int reps, double* ms_per_launch, d
  * 0.002; negative: the plain Galerkin operator. */
 #define MM_OPT_SA_FILTER_E6 20
 /* MM_OPT_ONE_LAUNCH: blocks of a demag solve's persistent launch (MM_OPT_GRAPH) at most; each holds an SM until the
- * solve has converged.  -1 (default): every SM; a third of them beside one or two other solves or minimizations in
- * flight on the device; no such launch beside more.  0: never such a launch, but separate kernels, between which
+ * solve has converged.  -1 (default): every SM; beside one or two other solves or minimizations in flight on the
+ * device its share of them, up to 98,304 nodes; else no such launch.  0: never such a launch, but separate kernels, between which
  * other streams' work runs.  The same results either way, bit for bit. */
 #define MM_OPT_ONE_LAUNCH 21
 int mm_set_option(mm_problem* h, int option, int value);

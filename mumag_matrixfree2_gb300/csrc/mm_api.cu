@@ -1316,19 +1316,22 @@ bool persistent_ok(mm_problem* h, SolverT<T>& F) {
 }
 
 // One solve, minimization or autotuning in flight.  Their number on the device decides how each runs its PCG, so that
-// several threads' problems share the GPU: alone on every SM, with one or two others on a third of them each,
-// and with more as separate kernels, whose many small launches overlap (48 particles on 16 threads, FP32
-// V-cycle: 16.3 s with every SM for each, 13.2 s with a cluster of 16 blocks each, 11.1 s as separate kernels, now
-// 10.2).  The cap holds for the call: outside one there is none to use.
+// several threads' problems share the GPU: alone on every SM; beside one or two others on its share of them, up to 96Ki
+// rows; else as separate kernels, whose many small launches overlap.  us a solve of two and of three threads, on shares
+// and as separate kernels (FP64): 50,653 rows 367 and 548, 313 and 440; 91,125 rows 572 and 733, 522 and 539; 125,000 rows
+// 794 and 810, 655 and 632; 357,911 rows 1556 and 1487, 1365 and 1205.  48 particles on 16 threads, FP32 V-cycle: 16.3 s
+// with every SM for each, 13.2 s with a cluster of 16 blocks each, 10.2 s as separate kernels.  The cap holds for the
+// call: outside one there is none to use.
 // The results are the same bits.
 std::atomic<int> g_solving[64];
+constexpr int SHARE_ROWS = 98304;
 
 struct SolveScope {
   mm_problem* const h;
   std::atomic<int>& n;
   explicit SolveScope(mm_problem* p) : h(p), n(g_solving[std::min(std::max(p->device, 0), 63)]) {
     const int k = ++n;
-    h->pcg_cap = k == 1 ? h->coop_sms : k <= 3 ? h->coop_sms / 3 : 0;
+    h->pcg_cap = k == 1 ? h->coop_sms : k <= 3 && h->N <= SHARE_ROWS ? h->coop_sms / k : 0;
     if (h->one_launch >= 0) h->pcg_cap = std::min(h->pcg_cap, h->one_launch);
   }
   ~SolveScope() {

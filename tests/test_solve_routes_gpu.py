@@ -287,3 +287,32 @@ def test_dealt_out_rows_against_compressed_rows(cuda_ok, precision):
             assert prob.get_option("coarse_cycle") == cycle and out[3] == 0
             ref = ref or out
             assert out[1:] == ref[1:] and np.array_equal(out[0], ref[0]), (lanes, graph, cycle)
+
+
+@pytest.mark.parametrize("workload, shares", [("cube40_h2_air200", True), ("cube80_h1.6_air200", False)])
+def test_a_solve_beside_another_problem(cuda_ok, workload, shares):
+    """Beside one other problem in flight a solve of 59,319 rows takes its share of the SMs in one launch, and one of
+    357,911 rows separate kernels, as it always did; the potential has the same bits."""
+    s, prob = _problem(workload)
+    m = syn.initial_state(s.N, seed=23, amplitude=0.3)
+    ref, alone = _launches(prob, m, np.zeros(s.N), 1e-10)
+    so, po = _problem("cube16_h2_air48")
+    mo = syn.initial_state(so.N, seed=24, amplitude=0.3)
+    stop, gate = threading.Event(), threading.Barrier(2)
+
+    def work():
+        gate.wait()
+        while not stop.is_set():
+            po.minimize(np.array([0.0, 0.0, -0.3]), mo, np.zeros(so.N), MinimizerParams(max_iter=200, tau_f=1e-14))
+
+    t = threading.Thread(target=work)
+    t.start()
+    gate.wait()
+    counts = set()
+    for _ in range(40):
+        out, n = _launches(prob, m, np.zeros(s.N), 1e-10)
+        counts.add(n)
+        assert out[1:] == ref[1:] and np.array_equal(out[0], ref[0])
+    stop.set()
+    t.join()
+    assert (max(counts) == alone) == shares, (counts, alone)
