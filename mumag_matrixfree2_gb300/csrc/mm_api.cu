@@ -281,6 +281,7 @@ struct mm_problem {
   float *d_r32 = nullptr, *d_d32 = nullptr;
   double* d_part = nullptr;      // NRED x MAXG block partials (shared by every reduction)
   mmk::PBar* d_pbar = nullptr;   // the one-launch PCG's grid barrier
+  int sms = 0;                   // of the device
   int coop_sms = 0;              // blocks of the one-launch PCG that the device can hold at once
   bool pcg_clusters = false;     // and whether a cluster of them
   int pcg_cap = 0;               // blocks of the one-launch PCG at most in this call (SolveScope)
@@ -1607,16 +1608,23 @@ void run_pcg_mp(mm_problem* h, double tol, int maxiter, int* iters, double* r2_o
   if (r2_out) *r2_out = h->h_sc->red[R_R2];
 }
 
-// Lanes a row of the FP64 right-hand side and energy below this many magnetic rows (one from there on): an energy
-// evaluation with 1, 2, 4 and 8 lanes takes 66, 54, 51 and 54 us (9k rows), 62, 56, 51 and 53 (3k); 102 and 114 with 1
-// and 2 lanes (133k).  The right-hand side of a solve with 1 and 4 lanes: 626 and 618 us a solve (9k rows).
-constexpr int OP_LANES = 4;
-constexpr int OP_LANES_ROWS = 65536;
+// Lanes a row of the FP64 energy: four, else two, as long as that gives no SM a second block, whose FP64 operations would
+// wait for the first's (ends of the ranges: 9,728 and 19,456 magnetic rows).  The kernel with 1, 2 and 4 lanes, cold:
+// 9,261 rows 26.8, 22.4 and 20.2 us; 12,167 rows 27.2, 22.6 and 23.7; 17,576 rows 27.7, 22.7 and 24.3; 19,683 rows 27.7, 27.9
+// and 29.1; 39,304 rows 31.1, 37.1 and 41.4; 64,000 rows 39.0, 46.4 and 53.7.
+int energy_lanes(const mm_problem* h) {
+  const int n = h->eops.n_rows;
+  return grid_rows(n, 4) <= h->sms ? 4 : grid_rows(n, 2) <= h->sms ? 2 : 1;
+}
 
-// b = D m on the magnetic rows; lanes a row as in enqueue_energy
+// b = D m on the magnetic rows, by four lanes a row where that gives loads in flight that are missing otherwise.  The kernel
+// with 1 and 4 lanes, cold: 9,261 rows 21.6 and 12.2 us; 39,304 rows 22.6 and 15.2; 74,088 rows 23.1 and 19.8; 97,336 rows
+// 24.7 and 24.8; 132,651 rows 27.5 and 29.7.
+constexpr int RHS_LANES_ROWS = 65536;
+
 void rhs_rows(mm_problem* h, const double* m) {
   const int n = h->eops.n_rows;
-  if (n < OP_LANES_ROWS) mmk::k_rhs_s<OP_LANES><<<grid_rows(n, OP_LANES), BS, 0, h->st>>>(h->eops, m, h->d_b);
+  if (n < RHS_LANES_ROWS) mmk::k_rhs_s<4><<<grid_rows(n, 4), BS, 0, h->st>>>(h->eops, m, h->d_b);
   else mmk::k_rhs_s<1><<<grid_elem(n), BS, 0, h->st>>>(h->eops, m, h->d_b);
   LAUNCH_CHECK();
 }
@@ -1787,8 +1795,11 @@ void enqueue_energy(mm_problem* h, const double* d_m, const double* d_U, const d
                                  h->d_part);
   };
   const int n = h->eops.n_rows;
-  if (n < OP_LANES_ROWS) fp64(mmk::k_energy_grad_s<OP_LANES>, grid_rows(n, OP_LANES));
-  else fp64(mmk::k_energy_grad_s<1>, grid_elem(n));
+  switch (energy_lanes(h)) {
+    case 4: fp64(mmk::k_energy_grad_s<4>, grid_rows(n, 4)); break;
+    case 2: fp64(mmk::k_energy_grad_s<2>, grid_rows(n, 2)); break;
+    default: fp64(mmk::k_energy_grad_s<1>, grid_elem(n));
+  }
   LAUNCH_CHECK();
 }
 
@@ -3620,6 +3631,7 @@ int mm_create(int N, int E, const int* conn, const double* volume, const double*
       CK(cudaGetDevice(&dev));
       CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
       if (sms > 0) g_vec_cap = std::min(4 * sms, MAXG);
+      h->sms = sms;
     }
     CK(cudaEventCreate(&h->ev0));
     CK(cudaEventCreate(&h->ev1));
