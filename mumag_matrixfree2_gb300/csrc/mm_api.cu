@@ -137,8 +137,9 @@ struct SolverT {
 };
 
 // Sizes whose PCG runs as one launch (V-cycle in T).  FP64: all measured (1,331 to 1,601,613 rows: 239 us a solve
-// against 469 as separate kernels, 5.83 against 6.69 ms).  FP32: up to 3/4 Mi rows (357,911 rows 1.55 against 1.78 ms;
-// 1,601,613 rows 5.17 against 4.96 ms: streaming FP32 operators wants the 2048 threads an SM of the separate kernels).
+// against 469 as separate kernels, 5.83 against 6.69 ms).  FP32: up to 3/4 Mi rows (778,688 rows 3.41 against 3.71 ms,
+// 1,000,000 rows 4.11 against 4.23; 1,331,000 rows 6.31 against 6.12, 1,601,613 rows 5.17 against 4.96: streaming FP32
+// operators wants the 2048 threads an SM of the separate kernels).
 template <class T>
 bool one_launch_rows(int64_t n) {
   return sizeof(T) == 8 || n <= 786432;
@@ -3294,13 +3295,15 @@ inline int fold_offset(int n) { return (n + 31) / 32 * 32; }
 
 // Levels whose prolongation and post-smoothing are folded into one product.  It has about half as many entries again
 // (17 against 10 a row on level 0, 56 against 37 on level 1) but saves a phase of the one-launch PCG (7k clocks and
-// more: a barrier and a chain of dependent loads), or a launch, and the pre-smoothed iterate.  A solve without, with
-// it on the levels from 1, and on all: 1,331 rows 306 and 267 us; 59,319 rows 726, 688 and 665 (FP32 V-cycle 677, 652
-// and 605); 357,911 rows 1833, 1805 and 1847 (1623, 1620 and 1659); 1,601,613 rows 5.97 and 5.88 ms (4.96 and 5.08,
-// where level 1 has 222,818 rows).
+// more: a barrier and a chain of dependent loads), or a launch, and the pre-smoothed iterate.  A solve in us without and
+// with level 0 folded, FP64 (FP32 V-cycle): 59,319 rows 626 and 572 (529, 491); 91,125 rows 724 and 679 (618, 577);
+// 103,823 rows 799 and 786 (727, 643); 110,592 rows 827 and 847 (704, 674); 117,649 rows 860 and 929 (724, 725); 125,000
+// rows 824 and 897 (679, 712).  Level 1, FP64: 262,144 rows 1759 and 1728, 636,056 rows 3170 and 3066, 1,601,613 rows (222,818
+// on level 1) 5970 and 5880; FP32: 300,763 rows 1536 and 1527, 357,911 rows (57,907) 1635 and 1650, 474,552 rows 2754 and
+// 2852.
 template <class T>
 bool fold_rows(int l, int64_t n) {
-  return n <= (l == 0 ? 131072 : sizeof(T) == 8 ? 262144 : 65536);
+  return n <= (sizeof(T) == 8 ? (l == 0 ? 106496 : 262144) : (l == 0 ? 116736 : 65536));
 }
 
 // fused coarse correction only where the dense factors stay small: Z = Ainv M costs nc^2 n host FLOPs, W and Z hold
