@@ -222,7 +222,8 @@ int mm_apply_A(mm_problem* h, const double* U, double* y);
 int mm_precond(mm_problem* h, const double* r, double* z);
 
 /* Demag solve: b = D m, PCG from U_inout to relative residual tol (recursive residual, as
- * src/poisson_solve.py:422-478), U_inout <- U.  rel_res = sqrt(r.r / b.b).
+ * src/poisson_solve.py:422-478), U_inout <- U.  rel_res = sqrt(r.r / b.b).  After an error U_inout holds no
+ * usable potential (mm_solve_u_dev iterates on it where it lies).
  * Returns MM_MAXITER when maxiter was reached first.
  * Replaces solve_U (src/poisson_solve.py:748-771) and the C++ solve_poisson
  * (src/cpp/cpp_mkl_minimizer.cpp:208-231). */
@@ -399,7 +400,8 @@ int mm_get_option(mm_problem* h, int option, int* value);
  * PCG iterations or whole V-cycles so that cache state and neighbours are those of a solve, and keeps the
  * fastest when it beats the heuristic's shape by more than 3 %; then times the V-cycle with and without the fused coarse correction in each solver and
  * sets MM_OPT_COARSE_FUSE accordingly.  CUDA events on the problem's stream, `reps`
- * launches per candidate.  A JSON report (candidates, times in microseconds, choices) is written to
+ * launches per candidate.  A JSON report (candidates, times in microseconds: `vcycle_us` holds those of a
+ * PCG iteration where the solves run as one launch, of a V-cycle else; choices) is written to
  * `report` (may be NULL; truncated to report_len - 1 characters).  No counterpart in the reference. */
 int mm_autotune(mm_problem* h, int reps, char* report, int report_len);
 

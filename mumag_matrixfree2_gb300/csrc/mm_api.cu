@@ -63,7 +63,7 @@ inline int grid_ilp(int64_t n) {
 }
 // warps (log2) of one chunk of the PCG's reductions over n rows (chunk_finish): one warp while the rows
 // give every SM fewer than 16 of them, else the block's eight
-inline int red_kshift(int64_t n) { return grid_ilp(n) * (BS / 32) < 2432 ? 0 : 3; }
+inline int red_kshift(int64_t n) { return grid_ilp(n) * (BS / 32) < 16 * mmk::TUNED_SMS ? 0 : 3; }
 inline int grid_rows(int64_t n, int tpr) {
   const int rpb = BS / tpr;
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + rpb - 1) / rpb, MAXG));
@@ -163,7 +163,7 @@ int choose_tpr(int64_t rows, int64_t nnz, int64_t n) {
     while (t < 32 && (rows * t < 262144) && t < avg) t *= 2;
     return t;
   }
-  const double per_sm = (double)rows / 152.0;
+  const double per_sm = (double)rows / mmk::TUNED_SMS;
   const double clocks = sizeof(T) == 8 ? 16.0 : 3.0;  // a warp's multiply-add or reduction step
   int best = 2;
   double best_cost = 1e300;
@@ -865,7 +865,7 @@ void level_operators(mm_problem* h, SolverT<T>& S, int l, F&& f, N&& f_not) {
   if (c.G.nnz > 0) go(on && g, c.G, h->g_host[l], "G");
 }
 
-// The layouts that the one-launch PCG reads, for the operators that it would read now; called wherever that changes
+// The dealt-out layouts that solves read, for the operators that it would read now; called wherever that changes
 // (never inside a capture).
 template <class T>
 void ensure_lanes(mm_problem* h, SolverT<T>& S) {
@@ -1217,9 +1217,9 @@ struct PcgPending {
   bool graph = false;
 };
 
-// the one-launch coarse cycle records a grid barrier that gave up waiting in the PCG's scalars
+// the one-launch PCG and the coarse cycle record a grid barrier that gave up waiting in the PCG's scalars
 void check_barrier(const mmk::Scalars* sc) {
-  if (sc->bar_err) throw Fail{MM_ERR_CUDA, "a grid barrier of the one-launch coarse cycle gave up waiting"};
+  if (sc->bar_err) throw Fail{MM_ERR_CUDA, "a grid barrier of a demag solve gave up waiting"};
 }
 
 void finish_pcg(mm_problem* h, const PcgPending& pend, int* iters, double* r2_out) {

@@ -20,6 +20,7 @@
 namespace mmk {
 
 constexpr int BS = 256;    // threads per block for every kernel here
+constexpr int TUNED_SMS = 152;  // SMs that the rules of layouts and reductions are measured for; launches ask the device
 constexpr int MAXG = 4096; // upper bound of any grid, and of the partials of one reduction
 
 enum RedSlot { R_BB0, R_BB, R_R2, R_RZ, R_PAP, R_SUM, R_E, R_MAX, R_A, R_B, R_C, R_D, NRED };
@@ -36,7 +37,7 @@ struct Scalars {
   int maxiter;
   int loops;        // graph-loop trips (hard stop for the conditional node)
   int rz_valid;     // 0 until the first r.z of a solve is reduced
-  int bar_err;      // a grid barrier of the one-launch coarse cycle gave up waiting (sticky)
+  int bar_err;      // a grid barrier of the one-launch PCG or of the coarse cycle gave up waiting (sticky)
   double red[NRED];
   unsigned cnt[NRED];
   // the minimizer's inner (preconditioner) solve, driven on the device

@@ -14,8 +14,8 @@
 // cache, and a phase of the 1,331-row mesh took 4 us.
 //
 // What bounds a phase now: below ~100k rows its barrier, the scalar that one thread forms (3 us, beside the first
-// loads) and a chain of three dependent loads; above, loads in flight (24 warps of 85 registers) against L2 and HBM
-// latency, with the FP64 pipe 30-40 % busy.  Deeper prefetching was slower: operators streamed to shared memory by a
+// loads) and a chain of three dependent loads; above, loads in flight (24 warps of 80 registers) against L2 and HBM
+// latency, with the FP64 pipe 41 % busy and HBM 28 % (357,911 rows), 53 and 47 % (1,601,613 rows).  Deeper prefetching was slower: operators streamed to shared memory by a
 // copying warp, prefetched to L2 one unit ahead, or shares dealt out in turn instead of contiguous.
 #pragma once
 

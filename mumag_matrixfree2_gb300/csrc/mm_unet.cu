@@ -785,6 +785,7 @@ const int TDEF[T_COUNT][2] = {{0, 16}, {0, 16}, {0, 16}, {1, 16}, {1, 32}, {1, 3
                               {1, 32}, {1, 32}, {1, 16}, {0, 16}, {0, 16}, {0, 16}};
 constexpr int IN_CH = 4;
 constexpr int NSPLIT_MAX = 64;
+constexpr int TUNED_SMS = 152;  // SMs that the splits and stages are measured for
 
 inline int nt_of(int cout) { return std::min(cout, 64); }
 // channels of a block of the weight gradient: 3 x 32 x 32 sums are 96 registers a thread
@@ -910,7 +911,7 @@ struct mm_unet {
     a.err = d_err;
     dim3 grid((unsigned)((v.t1 - v.t0 + 128 * mmn::MT - 1) / (128 * mmn::MT)), (unsigned)(cout / nt), (unsigned)nb);
     // more CTAs than SMs share them, and hide each other's copies
-    a.nst = mmn::conv_stages(v.P, cin, nt, grid.x * grid.y * grid.z <= 152 ? mmn::CONV_STAGES : 2);
+    a.nst = mmn::conv_stages(v.P, cin, nt, grid.x * grid.y * grid.z <= TUNED_SMS ? mmn::CONV_STAGES : 2);
     const size_t smem = 1024 + a.nst * mmn::conv_stage(v.P, nt);
     conv_dispatch(cin, nt, [&](auto kern) {
       allow_smem((const void*)kern);
@@ -925,7 +926,7 @@ struct mm_unet {
     const mmn::Vol& v = vol[d.level];
     const int range = v.t1 - v.t0, tiles = (range + mmn::WG_TV - 1) / mmn::WG_TV;
     const int blocks = 3 * (d.cin / wg_of(d.cin)) * (d.cout / wg_of(d.cout)) * nb;
-    ns = std::max(1, std::min({NSPLIT_MAX, tiles, 456 / blocks}));
+    ns = std::max(1, std::min({NSPLIT_MAX, tiles, 3 * TUNED_SMS / blocks}));
     const int per = (tiles + ns - 1) / ns;
     vpb = per * mmn::WG_TV;
     ns = (tiles + per - 1) / per;
@@ -961,7 +962,7 @@ struct mm_unet {
     });
     const int nw = 27 * d.cin * d.cout, n = nw + (train_bias ? d.cout : 0);
     int lg = 0;  // threads an element (log2): two blocks an SM
-    while (lg < 3 && (n << lg) < 304 * 256 && 2 << lg <= nb * ns) ++lg;
+    while (lg < 3 && (n << lg) < 2 * TUNED_SMS * 256 && 2 << lg <= nb * ns) ++lg;
     mmn::k_sum_parts<<<((n << lg) + 255) / 256, 256, 0, st_w>>>(part, nb * ns, lg, nw, n, d.cin, d.cout,
                                                               l == L_E0A ? IN_CH : d.cin, g + woff[l], g + boff[l]);
     UCK(cudaGetLastError());

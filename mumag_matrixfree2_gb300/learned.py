@@ -120,6 +120,7 @@ class UNet:
         return unflatten(flat)
 
     def get_grads(self) -> dict[str, np.ndarray]:
+        """The last backward pass's gradients by layer: parts of one array of this call (copy what is to be kept alone)."""
         flat = np.empty(self.n_params, np.float32)
         self._check("mm_unet_get_grads", _abi.lib().mm_unet_get_grads(self.h, _f32p(flat)))
         return unflatten(flat, copy=False)
