@@ -316,3 +316,34 @@ def test_a_solve_beside_another_problem(cuda_ok, workload, shares):
     stop.set()
     t.join()
     assert (max(counts) == alone) == shares, (counts, alone)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32_precond", "mixed"])
+def test_threads_solve_and_minimize_with_the_bits_of_one(cuda_ok, precision):
+    """Five threads at once, each solving and minimizing on a handle of its own: how many others are in flight changes the
+    form of a solve and of the minimizer's graph, not what they return."""
+    n = 5
+    handles = [_problem("cube16_h2_air48", precision) for _ in range(n)]
+    mp = MinimizerParams(max_iter=6, tau_f=1e-10, eps_a=1e-8, cg_tol=1e-10)
+
+    def both(k):
+        s, prob = handles[k]
+        m = syn.initial_state(s.N, seed=30 + k, amplitude=0.2)
+        U = prob.solve_u(m, np.zeros(s.N), 1e-10)
+        return (U[0], *U[1:3], *prob.minimize(np.array([0.0, 0.0, -0.3]), m, np.zeros(s.N), mp)[:2])
+
+    ref = [both(k) for k in range(n)]
+    bad, gate = [], threading.Barrier(n)
+
+    def work(k):
+        gate.wait()
+        for _ in range(4):
+            if not all(np.array_equal(a, b) for a, b in zip(both(k), ref[k])):
+                bad.append(k)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(n)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
