@@ -1701,12 +1701,14 @@ int solve_dev(mm_problem* h, const double* d_m, double* d_U, double tol, int max
   const bool zero_mean = !h->has_mask;
   const bool mixed = h->mixed && h->s32.built;
   const bool mp = !mixed && h->fp32_precond && h->s32.built && multilevel(h, h->s32);
+  CK(cudaEventRecord(h->ev0, h->st));
+  enqueue_rhs(h, d_m, false);
   // The one-launch PCG takes the caller's U as its iterate and forms b.b itself: two copies and an inner product
   // less in front of and behind it (10 us of a solve).  A U that its loads and stores cannot take is copied instead.
+  // (Looked up while the device forms the right-hand side.)
   const bool direct = !mixed && !zero_mean && iterable(h, d_U) &&
                       (mp ? persistent_ok(h, h->s32) && h->use_a0df() : persistent_ok(h, h->s64));
-  CK(cudaEventRecord(h->ev0, h->st));
-  enqueue_rhs(h, d_m, !direct);
+  if (!direct) dot(h, h->N, h->d_b, nullptr, R_BB0);
   if (x0_ready) CK(cudaStreamWaitEvent(h->st, x0_ready, 0));
   struct Iterate {  // s64.x for this call
     mm_problem* h;
