@@ -1095,15 +1095,15 @@ void enqueue_dir_step(mm_problem* h, SolverT<T>& S) {
   const int N = h->N;
   const double w = sizeof(T);
   auto& l0 = S.lv[0];
+  const bool ml = multilevel(h, S);
+  const int kshift = ml ? red_kshift(N) : 3;  // without a one launch to agree with, a block's partial: fewer to add up
   tagged<T>(h, MM_PROF_PCG_DIR, 0, mat_bytes(l0.A) + 5.0 * w * N, [&] {
-    launch(h, mmk::k_pcg_dir<T>, grid_ilp(N), BS, l0.A.s, S.z, S.p, S.Ap, S.sc, h->d_part,
-           red_kshift(N));
+    launch(h, mmk::k_pcg_dir<T>, grid_ilp(N), BS, l0.A.s, S.z, S.p, S.Ap, S.sc, h->d_part, kshift);
     LAUNCH_CHECK();
   });
-  const bool ml = multilevel(h, S);
   tagged<T>(h, MM_PROF_PCG_STEP, 0, (ml ? 8.0 : 6.0) * w * N, [&] {
     launch(h, mmk::k_pcg_step<T>, grid_ilp(N), BS, N, S.x, S.r, S.p, S.Ap, ml ? l0.s : nullptr, l0.x, S.sc,
-           h->d_part, red_kshift(N));
+           h->d_part, kshift);
     LAUNCH_CHECK();
   });
 }
@@ -1473,7 +1473,7 @@ void enqueue_pcg_start(mm_problem* h, SolverT<T>& S, double tol, int maxiter) {
   const double w = sizeof(T);
   tagged<T>(h, MM_PROF_INIT_RESIDUAL, 0, mat_bytes(l0.A) + 5.0 * w * N, [&] {
     launch(h, mmk::k_init_residual<T>, grid_ilp(N), BS, l0.A.s, S.x, S.b, S.r, ml ? l0.s : nullptr, l0.x, S.sc,
-           h->d_part, red_kshift(N));
+           h->d_part, ml ? red_kshift(N) : 3);
     LAUNCH_CHECK();
   });
   if (ml) enqueue_vcycle<T>(h, S, S.r, S.z, false, nullptr);
